@@ -276,10 +276,12 @@ def fp64_peak_errors(bits, runs, threads):
     return out
 
 
-# tensor-core MMA FLOPs per complex output point of the inverse transform,
-# by code length: the Good-Thomas stages 31 x 33 (Lc = 1023), 31 x 12 x 11
-# (4092) and 31 x 30 x 11 (10230) as real 2R x 2R GEMMs, 8 R per stage
-TC_MMA_FLOPS_PER_POINT = {1023: 8 * (31 + 33), 4092: 8 * (31 + 12 + 11), 10230: 8 * (31 + 30 + 11)}
+# tensor-core MMA FLOPs per complex output point of the inverse transform, by
+# code length: a step is M = 128 rows times (K1 = 80, 96, 112) x (N1 = 128, 192,
+# 192) for the DFT-33 / 44 / 55 and 64 x N1 for the DFT-31, padding included,
+# over 4 x 1023, 2 x 4092 or 10230 points
+TC_MMA_FLOPS_PER_POINT = {1023: 2 * 128 * 128 * (80 + 64) // 4092, 4092: 2 * 128 * 192 * (96 + 64) // 8184,
+                          10230: 2 * 128 * 192 * (112 + 64) // 10230}
 
 
 # index of a constellation's PRN inside its code-length group's row-peak
@@ -611,7 +613,7 @@ def main():
         against the measured sustained dense FP16/BF16 rate (it is timed
         inside a long step), the FP32 kernels against the FP32 pipe.  For the
         tensor-core kernel `tensor_pipe_util` is the fraction of that rate its
-        executed MMAs take (the DFT stages as dense real 2R x 2R GEMMs)."""
+        executed MMAs take (padding included)."""
         dname, (dms, dl, dfl) = max(agg.items(), key=lambda kv: kv[1][0])
         avg_launch_s = dms / dl / 1e3
         achieved = dfl / dl / avg_launch_s / 1e12
@@ -628,8 +630,8 @@ def main():
             executed = rows * SAMPLES_PER_CHIP * lc * TC_MMA_FLOPS_PER_POINT[lc]
             extra = {"tensor_pipe_util": executed / avg_launch_s / 1e12 / peak,
                      "executed_tflops": executed / avg_launch_s / 1e12,
-                     "executed_flops": "the DFT stages as dense real 2R x 2R GEMMs, 8 x (sum of the radices) per "
-                                       "complex output point (%d at Lc = %d)" % (TC_MMA_FLOPS_PER_POINT[lc], lc)}
+                     "executed_flops": "the MMAs of both GEMM stages with their padding: %d per complex output "
+                                       "point at Lc = %d" % (TC_MMA_FLOPS_PER_POINT[lc], lc)}
         else:
             peak = fp32_peak_tflops(sm_mhz)
             src = ("148 SM x 128 FP32 lanes x 2 flop x median SM clock under load (%.0f MHz); "

@@ -487,15 +487,16 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
       // reading the FP32 spectra back from memory)
       if (MODE == FWD_Z && p.z16) {
         using U = TcUnits<M>;
-        for (int e = tid; e < BC * U::PER_SEQ; e += NT) {
-          const int s = e / U::PER_SEQ, r = e - s * U::PER_SEQ;
+        for (int e = tid; e < BC * U::UNITS; e += NT) {
+          const int s = e / U::UNITS, r = e - s * U::UNITS;
           const int q = seq_of(s);
           if (q < 0) continue;
-          const uint2 m = __ldg(p.z16_map + r);
-          const unsigned off[4] = {m.x & 0xffffu, m.x >> 16, m.y & 0xffffu, m.y >> 16};
-          float2 v[4];
+          const uint4 m = __ldg(p.z16_map + r);
+          const unsigned off[8] = {m.x & 0xffffu, m.x >> 16, m.y & 0xffffu, m.y >> 16,
+                                   m.z & 0xffffu, m.z >> 16, m.w & 0xffffu, m.w >> 16};
+          float2 v[8];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
+          for (int i = 0; i < 8; ++i) {
             v[i] = make_float2(0.f, 0.f);
             if (off[i] != 0xffffu) {
               v[i] = buf[s * LC + (int)off[i]];
@@ -503,7 +504,8 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
               v[i].y *= p.z16_scale;
             }
           }
-          p.z16[(size_t)q * U::PER_SEQ + r] = pack_unit(v);
+          uint4* dst = p.z16 + (size_t)q * U::PER_SEQ + r;
+          pack_unit(v, dst[0], dst[U::UNITS]);
         }
         __syncthreads();
       }
@@ -642,13 +644,10 @@ cudaError_t launch_forward_z(const PolyClass& pc, int n_ab, float2* d_z, int num
 std::vector<uint16_t> tc_unit_map(int M) {
   auto build = [](auto u) {
     using U = decltype(u);
-    std::vector<uint16_t> t((size_t)U::PER_SEQ * 4);
-    for (int r = 0; r < U::PER_SEQ; ++r) {
-      const int j = r / U::ROWS1, row = r - j * U::ROWS1, kp = U::row_part(row);
-      for (int i = 0; i < 4; ++i) {
-        const int d1 = 4 * j + i;
-        t[(size_t)r * 4 + i] = d1 < 31 ? (uint16_t)U::src_offset(d1, kp) : (uint16_t)0xffffu;
-      }
+    std::vector<uint16_t> t((size_t)U::UNITS * 8);
+    for (int r = 0; r < U::UNITS; ++r) {
+      for (int i = 0; i < 8; ++i)
+        t[(size_t)r * 8 + i] = U::filled(r, i) ? (uint16_t)U::src_offset(r, i) : (uint16_t)0xffffu;
     }
     return t;
   };
@@ -665,7 +664,7 @@ cudaError_t launch_forward_z_tc(const PolyClass& pc, int n_ab, float2* d_z, void
   PfaParams p = {};
   p.z = d_z;
   p.z16 = static_cast<uint4*>(d_z16);
-  p.z16_map = static_cast<const uint2*>(d_map);
+  p.z16_map = static_cast<const uint4*>(d_map);
   p.z16_scale = z16_scale;
   p.n_seq = n_ab * 2 * pc.S;
   p.S = pc.S;
@@ -679,7 +678,7 @@ cudaError_t launch_forward_seqs_tc(const PolyClass& pc, long long n_seq, float2*
   PfaParams p = {};
   p.z = d_z;
   p.z16 = static_cast<uint4*>(d_z16);
-  p.z16_map = static_cast<const uint2*>(d_map);
+  p.z16_map = static_cast<const uint4*>(d_map);
   p.z16_scale = z16_scale;
   p.n_seq = (int)n_seq;
   p.S = pc.S;

@@ -120,12 +120,12 @@ cudaError_t launch_second_from_rows(const SearchDims& dims, int n_hyp, const flo
 // n_prn rows).  Keys are [ant][bin][hyp][prn].
 cudaError_t launch_tc_candidates(const SearchDims& dims, int n_hyp, const unsigned long long* d_keys, float keep,
                                  int2* d_cand, int* d_count, cudaStream_t st);
-// Tensor-core search: FP16 operands in the (31, R2, R3) frequency layout
-// (launch_tc_pack of Z and of the code spectra), then the three-stage tcgen05
+// Tensor-core search: FP16 operands in the (R1, 31, GR) frequency layout
+// (TcUnits; launch_tc_pack of the code spectra), then the two-stage tcgen05
 // correlator (FP32 accumulation in TMEM).  Keys hold |y|^2 scaled by 2^-2k
 // (comparisons only) and must be zeroed before the launch; *d_err is set
 // non-zero when a bounded wait on the tensor cores expired.
-size_t tc_operand_bytes(const PolyClass& pc, long long n_seq, bool code);
+size_t tc_operand_bytes(const PolyClass& pc, long long n_seq);
 // the three inverse-DFT matrices of class M in the correlator's shared-memory
 // layouts (FP16), to be uploaded once and passed as d_bmat
 std::vector<unsigned char> tc_dft_matrices(int M);

@@ -34,44 +34,58 @@ struct Geo {
   __device__ static __forceinline__ int offset(int a, int b, int c) { return a * COLS + c * 33 + b; }
 };
 
-// FP16 operands of the tensor-core search in its (31, R2, R3) frequency
-// layout (Lc = 31 R2 R3; (R2, R3) = (33, 1), (12, 11), (30, 11) for M = 1,
-// 4, 10).  Unit (seq, j, u), u = d3 R2 + d2, holds the spectrum at digits
-// (d1, d2, d3), d1 = 4j .. 4j + 3 (zero for d1 >= 31), as 4 half2 (16
-// bytes) split into real and imaginary parts: (re0, re1), (re2, re3),
-// (im0, im1), (im2, im3) (pack_unit), so that the products of two units
-// take four packed FP16 operations per pair of values and need no
-// repacking; the stage-1 operand rows keep this order of their K entries
-// and the stage-1 DFT matrix is built for it.  A frequency digit d of radix R stands for the natural
-// frequencies k = d (LC / R) (mod R); src_offset is where the FP32 engine's
-// digit layout [a][c][b] of the (31, 33, M) map holds the same frequency.
-__device__ __forceinline__ uint4 pack_unit(const float2 (&v)[4]) {
-  const __half2 a = __floats2half2_rn(v[0].x, v[1].x), b = __floats2half2_rn(v[2].x, v[3].x);
-  const __half2 c = __floats2half2_rn(v[0].y, v[1].y), d = __floats2half2_rn(v[2].y, v[3].y);
-  return make_uint4(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b),
-                    *reinterpret_cast<const uint32_t*>(&c), *reinterpret_cast<const uint32_t*>(&d));
+// FP16 operands of the tensor-core search.  Lc = R1 x 31 x GR with R1 = 33,
+// 44, 55 for M = 1, 4, 10; GR counts the digits left over (1; 3; 2 x 3).
+// Unit u = (gr 4 + j) R1P + d1 of a sequence holds the spectrum at 31-digits
+// 8 j .. 8 j + 7 (zero for digit 31), R1-digit d1 (zero from R1 on: R1P is R1
+// padded so that eight units from d1 = 0 on are 128 aligned bytes, one
+// shared-memory wavefront) and left-over digits gr
+// (M = 10: gr = 2 b + h, b of 3 and h of 2) as eight FP16 real parts (16
+// bytes, in the first plane of PER_SEQ / 2 units) and eight imaginary parts
+// (the same place in the second plane).  A unit is then one 16-byte row of
+// the first stage's operand (8 columns of one K entry), and the products of
+// two units are packed FP16 operations on whole registers.  A frequency
+// digit d of radix R stands for the natural frequencies k = d (Lc / R) (mod
+// R); src_offset is where the FP32 engine's digit layout [a][c][b] of the
+// (31, 33, M) map holds the same frequency.
+__device__ __forceinline__ void pack_unit(const float2 (&v)[8], uint4& re, uint4& im) {
+  uint32_t r[4], i[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const __half2 a = __floats2half2_rn(v[2 * k].x, v[2 * k + 1].x);
+    const __half2 b = __floats2half2_rn(v[2 * k].y, v[2 * k + 1].y);
+    r[k] = *reinterpret_cast<const uint32_t*>(&a);
+    i[k] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  re = make_uint4(r[0], r[1], r[2], r[3]);
+  im = make_uint4(i[0], i[1], i[2], i[3]);
 }
 
 template <int M>
 struct TcUnits {
-  static constexpr int R2 = M == 1 ? 33 : M == 4 ? 12 : 30, R3 = M == 1 ? 1 : 11;
-  static constexpr int LC = 1023 * M, ROWS1 = R2 * R3, PER_SEQ = 8 * ROWS1;
-  static constexpr int E1 = (LC / 31) * modinv_c((LC / 31) % 31, 31);
-  static constexpr int E2 = (LC / R2) * modinv_c((LC / R2) % R2, R2);
-  static constexpr int E3 = (LC / R3) * modinv_c((LC / R3) % R3, R3);
+  static constexpr int R1 = M == 1 ? 33 : M == 4 ? 44 : 55, GR = M == 1 ? 1 : M == 4 ? 3 : 6;
+  static constexpr int R1P = (2 * R1 + 15) / 16 * 8;  // 40, 48, 56
+  static constexpr int LC = 1023 * M, UNITS = GR * 4 * R1P, PER_SEQ = 2 * UNITS;
+  static_assert(R1 * 31 * GR == LC, "factorisation");
+  static constexpr int digit(int R) { return (LC / R) * modinv_c((LC / R) % R, R); }
   static constexpr int UB = modinv_c((LC / 33) % 33, 33);
   static constexpr int UC = M == 1 ? 0 : modinv_c((LC / M) % M, M);
   __host__ __device__ static constexpr int freq_part(int d, int R, int E) { return ((d * (LC / R)) % R) * E; }
-  // frequency contribution of the (d2, d3) digits of stage-1 row u
-  __host__ __device__ static __forceinline__ int row_part(int u) {
-    const int d3 = u / R2, d2 = u - d3 * R2;
-    return freq_part(d2, R2, E2) + freq_part(d3, R3, E3);
+  // 31-digit i of unit u holds a value (not padding)
+  __host__ __device__ static __forceinline__ bool filled(int u, int i) {
+    return u % R1P < R1 && 8 * ((u / R1P) & 3) + i < 31;
   }
-  // digit-layout offset [a][c][b] of slot d1 (< 31) of a row with row_part kp
-  __host__ __device__ static __forceinline__ int src_offset(int d1, int kp) {
-    const int k = (freq_part(d1, 31, E1) + kp) % LC;
+  // digit-layout offset of the frequency at 31-digit i of unit u
+  __host__ __device__ static __forceinline__ int src_offset(int u, int i) {
+    constexpr int E1 = digit(R1), E31 = digit(31), E3 = M == 1 ? 0 : digit(3), E2 = M == 10 ? digit(2) : 0;
+    const int q = u / R1P, d1 = u - q * R1P, gr = q >> 2, d2 = 8 * (q & 3) + i;
+    const int b = M == 10 ? gr >> 1 : gr, h = M == 10 ? gr & 1 : 0;
+    int k = freq_part(d1, R1, E1) + freq_part(d2, 31, E31);
+    if (M != 1) k += freq_part(b, 3, E3);
+    if (M == 10) k += freq_part(h, 2, E2);
+    k %= LC;
     const int kb = (UB * k) % 33, kc = M == 1 ? 0 : (UC * k) % M;
-    return d1 * 33 * M + kc * 33 + kb;
+    return d2 * 33 * M + kc * 33 + kb;  // the 31-digit is the same in both layouts
   }
 };
 
@@ -122,7 +136,7 @@ struct PfaParams {
   float* p2rows;              // CAND (optional): each listed row's second peak
                               // against its own maximum, where its key goes
   uint4* z16;                 // FWD_Z (optional): the transformed sequences also as TcUnits, x z16_scale
-  const uint2* z16_map;       // per unit: the 4 src_offset values as 16-bit fields (0xffff: zero)
+  const uint4* z16_map;       // per unit: the 8 src_offset values as 16-bit fields (0xffff: zero)
   float z16_scale;
 };
 

@@ -522,8 +522,8 @@ GroupBufs prepare_group(tga_ctx* ctx, const ClassGroup& grp, int n_ant, int nb, 
   if (ctx->precision == TGA_PRECISION_FP16_TC) {
     b.err = (int*)ctx->buf("tc.err", sizeof(int));
     const long long n_zseq = (long long)n_ab * 2 * pc.S;
-    b.z16 = ctx->buf(tag + ".z16", tc_operand_bytes(pc, n_zseq, false));
-    b.d16 = ctx->buf(tag + ".d16", tc_operand_bytes(pc, (long long)n_prn * 2, true));
+    b.z16 = ctx->buf(tag + ".z16", tc_operand_bytes(pc, n_zseq));
+    b.d16 = ctx->buf(tag + ".d16", tc_operand_bytes(pc, (long long)n_prn * 2));
     b.keys32 = (unsigned long long*)ctx->buf(tag + ".keys32", (size_t)n_ab * 2 * n_prn * sizeof(unsigned long long));
     b.p2rows = (float*)ctx->buf(tag + ".p2rows", (size_t)n_ab * 2 * n_prn * sizeof(float));
     b.cand = (int2*)ctx->buf(tag + ".cand", (size_t)n_ab * 2 * n_prn * sizeof(int2));
@@ -2055,10 +2055,10 @@ void nc_run_group(tga_ctx* ctx, const uint8_t* d_bits, size_t row_bytes, const d
   const int cw = chip_width_of(fs);
   const bool rows_p2 = tc && (2 * cw + pc.S) / pc.S <= 3;
   if (tc) {
-    d_z16 = ctx->buf("nc.z16", tc_operand_bytes(pc, n_seq, false));
+    d_z16 = ctx->buf("nc.z16", tc_operand_bytes(pc, n_seq));
     d_zmap = tc_unit_map_buf(ctx, pc.M);
     d_err = (int*)ctx->buf("tc.err", sizeof(int));
-    d_d16 = ctx->buf(tag + ".d16", tc_operand_bytes(pc, (long long)n_prn * 2, true));
+    d_d16 = ctx->buf(tag + ".d16", tc_operand_bytes(pc, (long long)n_prn * 2));
     const std::string mat_name = "tcmat." + std::to_string(pc.M);
     if (!ctx->uploaded.count(mat_name)) {
       const std::vector<unsigned char> mats = tc_dft_matrices(pc.M);
