@@ -180,18 +180,37 @@ cudaError_t launch_fine_sums(const uint8_t* d_bits, int n_ant, size_t row_bytes,
 // narrowband RFI scan of every antenna row (rfi.rs:91-168): f64 spectrum,
 // exact median bin power, local maxima above 15 dB (up to cap per antenna,
 // d_count counts all), exact autocorrelation popcounts at lags 1, 3, 16
-cudaError_t rfi_scan_device(const uint8_t* d_bits, int n_ant, size_t row_bytes, const double* d_mean, double* d_z,
-                            void* d_X, void* d_work, double* d_p, unsigned* d_hist, unsigned long long* d_prefix,
-                            unsigned long long* d_rank, int cap, unsigned* d_count, long long* d_bins,
-                            double* d_excess, unsigned long long* d_acf, int num_sms, cudaStream_t st,
-                            std::string* why);
+//
+// The median is a radix select over the powers' bit patterns (non-negative
+// doubles): two digits of 13 bits over all bins, then the bins that share both
+// (about 2^-14 of them) in a list of at most kRfiList, and the exact rank in it.
+constexpr int kRfiDigits = 1 << 13, kRfiShift0 = 50, kRfiShift1 = 37, kRfiList = 2048;
+struct RfiBufs {
+  double* z;                    // [n_ant][n] (FFT)
+  void* X;                      // [n_ant][n / 2] complex (FFT)
+  void* work;                   // fft64_workspace_bytes
+  double* p;                    // [n_ant][n / 2] bin powers
+  unsigned* hist;               // [n_ant][2][kRfiDigits]
+  unsigned long long* prefix;   // [n_ant]: the digits found, in the end the median's bits
+  unsigned* rank;               // [n_ant]: rank among the bins that share the prefix
+  unsigned* n_list;             // [n_ant]
+  unsigned long long* list;     // [n_ant][kRfiList]
+  unsigned* count;              // [n_ant] candidate lines found
+  long long* bins;              // [n_ant][cap]
+  double* excess;               // [n_ant][cap]
+  unsigned long long* acf;      // [n_ant][9]
+};
+cudaError_t rfi_scan_device(const uint8_t* d_bits, int n_ant, size_t row_bytes, const double* d_mean, const RfiBufs& b,
+                            int cap, int num_sms, cudaStream_t st, std::string* why);
 
-// f64 spectrum of `batch` real records of n samples (n even) held as doubles
-// in d_x (overwritten): p[a][k] = |X_a[k]|^2 for k < n / 2.  d_buf holds
-// batch * n / 2 complex doubles, d_work fft64_workspace_bytes(n, batch).
+// f64 spectrum of `batch` rows of packed bits (n = 8 row_bytes samples +-1 -
+// mean): p[a][k] = |X_a[k]|^2 for k < n / 2, and the histogram of their top
+// digits added to hist[a][0].  d_x holds batch * n doubles, d_buf batch * n / 2
+// complex doubles, d_work fft64_workspace_bytes(n, batch).
 size_t fft64_workspace_bytes(long long n, int batch);
-cudaError_t real_power_spectrum(double* d_x, void* d_buf, void* d_work, long long n, int batch, double* d_p,
-                                int num_sms, cudaStream_t st, std::string* why);
+cudaError_t real_power_spectrum(const uint8_t* d_bits, size_t row_bytes, const double* d_mean, double* d_x, void* d_buf,
+                                void* d_work, int batch, double* d_p, unsigned* d_hist, int num_sms, cudaStream_t st,
+                                std::string* why);
 
 // ACR Monte Carlo synthesizer (examples/gen_acr_tables.rs): n_points x
 // n_trials rows of 2 * period one-bit samples, packed MSB-first

@@ -8,12 +8,18 @@
 //   out[q Ns R + r Ns + k] = sum_{s < R} in[q Ns + k + s L / R] W_L^{s (k + r Ns) L / (Ns R)}
 //
 // (k < Ns, r < R, W_L = exp(-2 pi i / L)), so after the passes of all
-// factors of L the result is in natural order.  Powers of two run as
-// radix-16/8/4/2 butterflies, one per thread; other prime factors (up to
-// kMaxRadix) as one output per thread, an R-term sum.  Twiddles come from one
-// table W_L^m, m < L, built in double precision with sincospi.  A length
-// with a prime factor above kMaxRadix is transformed by Bluestein's chirp-z
-// identity over a power-of-two convolution.
+// factors of L the result is in natural order.  Each pass reads and writes
+// the whole batch, so what bounds a pass is HBM and what counts is their
+// number: the factors are gathered into radices of up to 33 (32; 33 = 3 x 11
+// and 15 = 3 x 5 without twiddles; 25; 31, ...), one whole butterfly per thread in
+// registers, and the first pass reads the packed bits themselves.  24 rows of
+// 1636800 samples (L = 32 x 25 x 33 x 31): the seven passes of radices 16, 2,
+// 3, 5, 5, 11, 31 with R-term sums took 4.2 ms, the four passes 0.41 ms.
+// Other prime factors up to kMaxRadix run as one output per thread, an R-term
+// sum.  Twiddles come from one table W_L^m, m < L, built in double precision
+// with sincospi; a butterfly loads about 2 sqrt(R) of them and forms the
+// others as products of two.  A length with a prime factor above kMaxRadix is
+// transformed by Bluestein's chirp-z identity over a power-of-two convolution.
 //
 // The real record of n samples is transformed as n/2 complex points z[m] =
 // x[2m] + i x[2m+1] (the layout the record already has as doubles), then
@@ -21,10 +27,12 @@
 // L = n/2, of which the scan keeps |X[k]|^2 for k < n/2.
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 #include <string>
 #include <vector>
 
+#include "dft64_consts.cuh"
 #include "engine.h"
 
 namespace tga {
@@ -46,36 +54,173 @@ __global__ void twiddle64_kernel(double2* __restrict__ tw, long long L) {
   }
 }
 
-// One pass of power-of-two radix R, one butterfly (R outputs) per thread.
-template <int R>
-__global__ void __launch_bounds__(256) pass_pow2_kernel(const double2* __restrict__ in, double2* __restrict__ out,
-                                                        const double2* __restrict__ tw, long long L, long long Ns,
-                                                        long long total_j) {
-  const long long LR = L / R, NsR = Ns * R, step = L / NsR;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total_j;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long a = t / LR, j = t - a * LR;
-    const long long k = j % Ns, q = j / Ns;
-    const double2* x = in + a * L + j;
-    double2 v[R];
+template <int R> __device__ __forceinline__ double kcosd(int m);
+template <int R> __device__ __forceinline__ double ksind(int m);
+#define TGA_D64(R)                                                                        \
+  template <> __device__ __forceinline__ double kcosd<R>(int m) { return kCosD##R[m]; } \
+  template <> __device__ __forceinline__ double ksind<R>(int m) { return kSinD##R[m]; }
+TGA_D64(3)
+TGA_D64(5)
+TGA_D64(7)
+TGA_D64(11)
+TGA_D64(13)
+TGA_D64(25)
+TGA_D64(31)
+TGA_D64(32)
+#undef TGA_D64
+
+// Forward DFTs of register arrays, outputs streamed to st(k, value).
+// Odd prime R: pairs s_n = x_n + x_{R-n}, d_n = x_n - x_{R-n} halve the terms.
+template <int R, class St>
+__device__ __forceinline__ void dft64_prime(const double2 (&x)[R], St&& st) {
+  constexpr int H = (R - 1) / 2;
+  double2 s[H], d[H];
 #pragma unroll
-    for (int s = 0; s < R; ++s) {
-      const double2 u = x[s * LR];
-      v[s] = s == 0 ? u : cmul64(u, __ldg(tw + (s * k * step) % L));
+  for (int n = 1; n <= H; ++n) {
+    s[n - 1] = make_double2(x[n].x + x[R - n].x, x[n].y + x[R - n].y);
+    d[n - 1] = make_double2(x[n].x - x[R - n].x, x[n].y - x[R - n].y);
+  }
+  double2 X0 = x[0];
+#pragma unroll
+  for (int n = 0; n < H; ++n) X0 = make_double2(X0.x + s[n].x, X0.y + s[n].y);
+  const double2 x0 = x[0];
+  st(0, X0);
+#pragma unroll
+  for (int k = 1; k <= H; ++k) {
+    double2 A = x0, B = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int n = 1; n <= H; ++n) {
+      const double c = kcosd<R>((n * k) % R), sn = ksind<R>((n * k) % R);
+      A.x = fma(s[n - 1].x, c, A.x);
+      A.y = fma(s[n - 1].y, c, A.y);
+      B.x = fma(d[n - 1].x, sn, B.x);
+      B.y = fma(d[n - 1].y, sn, B.y);
     }
-    // DFT-R of v: W_R^{r s} = tw[(r s mod R) L / R]
-    double2* y = out + a * L + q * NsR + k;
+    st(k, make_double2(A.x + B.y, A.y - B.x));      // A - i B
+    st(R - k, make_double2(A.x - B.y, A.y + B.x));  // A + i B
+  }
+}
+
+// N a power of two up to 32: decimation in time over x[off + i stride]
+template <int N, int STRIDE, int M>
+__device__ __forceinline__ void dft64_pow2(const double2 (&x)[M], int off, double2 (&y)[N]) {
+  if constexpr (N == 1) {
+    y[0] = x[off];
+  } else {
+    double2 e[N / 2], o[N / 2];
+    dft64_pow2<N / 2, 2 * STRIDE>(x, off, e);
+    dft64_pow2<N / 2, 2 * STRIDE>(x, off + STRIDE, o);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      double2 acc = v[0];
+    for (int k = 0; k < N / 2; ++k) {
+      double2 t = o[k];
+      if (4 * k == N)
+        t = make_double2(o[k].y, -o[k].x);  // times -i
+      else if (k > 0)
+        t = cmul64(o[k], make_double2(kcosd<32>(k * (32 / N)), -ksind<32>(k * (32 / N))));
+      y[k] = make_double2(e[k].x + t.x, e[k].y + t.y);
+      y[k + N / 2] = make_double2(e[k].x - t.x, e[k].y - t.y);
+    }
+  }
+}
+
+template <int R, class St>
+__device__ __forceinline__ void dft64(const double2 (&x)[R], St&& st) {
+  if constexpr ((R & (R - 1)) == 0) {
+    double2 y[R];
+    dft64_pow2<R, 1>(x, 0, y);
 #pragma unroll
-      for (int s = 1; s < R; ++s) {
-        const double2 w = __ldg(tw + ((r * s) % R) * LR);
-        acc.x += v[s].x * w.x - v[s].y * w.y;
-        acc.y += v[s].x * w.y + v[s].y * w.x;
+    for (int k = 0; k < R; ++k) st(k, y[k]);
+  } else if constexpr (R == 33 || R == 15) {
+    // 3 x P, coprime: n = (P n1 + 3 n2) mod R, k = (P (P^-1 mod 3) k1 + 3 (3^-1 mod P) k2) mod R
+    constexpr int P = R / 3, E1 = P * (P % 3 == 1 ? 1 : 2), E2 = 3 * (P == 11 ? 4 : 2);
+    double2 u[3][P];
+#pragma unroll
+    for (int n2 = 0; n2 < P; ++n2) {
+      const double2 t[3] = {x[(3 * n2) % R], x[(P + 3 * n2) % R], x[(2 * P + 3 * n2) % R]};
+      dft64_prime<3>(t, [&](int k1, double2 v) { u[k1][n2] = v; });
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1)
+      dft64_prime<P>(u[k1], [&](int k2, double2 v) { st((E1 * k1 + E2 * k2) % R, v); });
+  } else if constexpr (R == 25) {
+    // n = 5 n1 + n2, k = k1 + 5 k2, twiddles W_25^{n2 k1}
+    double2 u[5][5];  // [k1][n2]
+#pragma unroll
+    for (int n2 = 0; n2 < 5; ++n2) {
+      const double2 t[5] = {x[n2], x[5 + n2], x[10 + n2], x[15 + n2], x[20 + n2]};
+      dft64_prime<5>(t, [&](int k1, double2 v) {
+        u[k1][n2] = k1 * n2 == 0 ? v : cmul64(v, make_double2(kcosd<25>(k1 * n2), -ksind<25>(k1 * n2)));
+      });
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 5; ++k1) dft64_prime<5>(u[k1], [&](int k2, double2 v) { st(k1 + 5 * k2, v); });
+  } else {
+    dft64_prime<R>(x, st);
+  }
+}
+
+// One pass of radix R, one butterfly per thread; blockIdx.y is the sequence.
+// FIRST (Ns = 1): the input is the row's samples, complex point m = (sample
+// 2 m) + i (sample 2 m + 1), each +-1 - mean; a thread's R outputs are
+// contiguous, so the block's go out through shared memory in order.
+struct FirstSource {
+  const uint8_t* bits;
+  size_t row_bytes;
+  const double* mean;
+};
+constexpr int kPassThreads = 128;
+
+template <int R, bool FIRST>
+__global__ void __launch_bounds__(kPassThreads) pass64_kernel(const double2* __restrict__ in, FirstSource src,
+                                                              double2* __restrict__ out,
+                                                              const double2* __restrict__ tw, unsigned L,
+                                                              unsigned Ns) {
+  extern __shared__ double2 s_out[];
+  const unsigned LR = L / R, j = blockIdx.x * kPassThreads + threadIdx.x;
+  const size_t seq = (size_t)blockIdx.y * L;
+  double2 v[R];
+  if (j < LR) {
+    if constexpr (FIRST) {
+      const uint8_t* row = src.bits + (size_t)blockIdx.y * src.row_bytes;
+      const double m = src.mean[blockIdx.y], hi = 1.0 - m, lo = -1.0 - m;
+#pragma unroll
+      for (int s = 0; s < R; ++s) {
+        const unsigned i = j + s * LR;  // samples 2 i and 2 i + 1
+        const unsigned two = (unsigned)__ldg(row + (i >> 2)) >> (6 - 2 * (i & 3u));
+        v[s] = make_double2(two & 2u ? hi : lo, two & 1u ? hi : lo);
       }
-      y[r * Ns] = acc;
+      double2* o = s_out + threadIdx.x * (R + 1);
+      dft64<R>(v, [&](int r, double2 y) { o[r] = y; });
+    } else {
+      const unsigned q = j / Ns, k = j - q * Ns, b = k * (L / (Ns * R));  // twiddle of s: W_L^{s b}
+      const double2* x = in + seq + j;
+#pragma unroll
+      for (int s = 0; s < R; ++s) v[s] = x[(size_t)s * LR];
+      // W^{s b} = W^{(s % G) b} W^{(s - s % G) b}
+      constexpr int G = R <= 4 ? R : R <= 9 ? 3 : R <= 16 ? 4 : 6;
+      double2 lowp[G];
+#pragma unroll
+      for (int s = 1; s < G; ++s) lowp[s] = __ldg(tw + (size_t)s * b);
+#pragma unroll
+      for (int g = 0; g < R; g += G) {
+        double2 h = make_double2(1.0, 0.0);
+        if (g > 0) h = __ldg(tw + (size_t)g * b);
+#pragma unroll
+        for (int s = 0; s < G; ++s) {
+          if (g + s >= R || g + s == 0) continue;
+          const double2 w = s == 0 ? h : g == 0 ? lowp[s] : cmul64(h, lowp[s]);
+          v[g + s] = cmul64(v[g + s], w);
+        }
+      }
+      double2* y = out + seq + (size_t)q * Ns * R + k;
+      dft64<R>(v, [&](int r, double2 t) { y[(size_t)r * Ns] = t; });
     }
+  }
+  if constexpr (FIRST) {
+    __syncthreads();
+    const unsigned j0 = blockIdx.x * kPassThreads, n = min((unsigned)kPassThreads, LR - j0) * R;
+    double2* y = out + seq + (size_t)j0 * R;
+    for (unsigned i = threadIdx.x; i < n; i += kPassThreads) y[i] = s_out[i + i / R];
   }
 }
 
@@ -103,8 +248,9 @@ __global__ void __launch_bounds__(256) pass_any_kernel(const double2* __restrict
   }
 }
 
-// factors of L in pass order: 16, 8, 4, 2 for the power of two, then the
-// odd primes ascending; false when a prime factor exceeds kMaxRadix
+// radices of L in pass order: the power of two in as few parts of at most 32
+// as there can be, then the odd primes, 3 with 11 or 5 and 5 with 5 together;
+// false when a prime factor exceeds kMaxRadix
 bool factorise(long long L, std::vector<int>* radices) {
   radices->clear();
   long long m = L;
@@ -113,22 +259,38 @@ bool factorise(long long L, std::vector<int>* radices) {
     m /= 2;
     ++twos;
   }
-  while (twos >= 4) {
-    radices->push_back(16);
-    twos -= 4;
+  for (int parts = (twos + 4) / 5; parts > 0; --parts) {
+    const int t = (twos + parts - 1) / parts;
+    radices->push_back(1 << t);
+    twos -= t;
   }
-  if (twos == 3) radices->push_back(8);
-  if (twos == 2) radices->push_back(4);
-  if (twos == 1) radices->push_back(2);
+  std::vector<int> odd;
   for (long long p = 3; p * p <= m || m > 1; p += 2) {
     if (p * p > m) p = m;  // m is prime
     while (m % p == 0) {
       if (p > kMaxRadix) return false;
-      radices->push_back((int)p);
+      odd.push_back((int)p);
       m /= p;
     }
     if (m == 1) break;
   }
+  auto pair = [&](int p, int q) {
+    for (;;) {
+      size_t i = odd.size(), k = odd.size();
+      for (size_t t = 0; t < odd.size(); ++t) {
+        if (odd[t] == p && i == odd.size()) i = t;
+        else if (odd[t] == q) k = t;
+      }
+      if (i == odd.size() || k == odd.size()) return;
+      odd.erase(odd.begin() + (i > k ? i : k));
+      odd.erase(odd.begin() + (i > k ? k : i));
+      radices->push_back(p * q);
+    }
+  };
+  pair(5, 5);
+  pair(3, 11);
+  pair(3, 5);
+  for (int p : odd) radices->push_back(p);
   return true;
 }
 
@@ -138,30 +300,61 @@ int grid_for(long long work, int num_sms) {
   return (int)(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
-// Stockham passes over `batch` sequences of length L in a (ping-pong with
-// b); returns the buffer holding the result.
-double2* stockham(double2* a, double2* b, const double2* tw, long long L, int batch, const std::vector<int>& radices,
-                  int num_sms, cudaStream_t st, cudaError_t* err) {
+template <int R, bool FIRST>
+cudaError_t run_pass64(const double2* x, const FirstSource& src, double2* y, const double2* tw, long long L, int batch,
+                       long long Ns, cudaStream_t st) {
+  const size_t smem = FIRST ? (size_t)kPassThreads * (R + 1) * sizeof(double2) : 0;
+  auto kern = pass64_kernel<R, FIRST>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 grid((unsigned)((L / R + kPassThreads - 1) / kPassThreads), (unsigned)batch);
+  kern<<<grid, kPassThreads, smem, st>>>(x, src, y, tw, (unsigned)L, (unsigned)Ns);
+  return cudaGetLastError();
+}
+
+// Stockham passes over `batch` sequences of length L (below 2^30) in a
+// (ping-pong with b); *result is the buffer holding the result.  With src the
+// first pass reads the rows' bits and a is only written.
+cudaError_t stockham(double2* a, double2* b, const FirstSource* src, const double2* tw, long long L, int batch,
+                     const std::vector<int>& radices, int num_sms, cudaStream_t st, double2** result) {
   long long Ns = 1;
   double2* x = a;
   double2* y = b;
+  const FirstSource none = {};
   for (int R : radices) {
-    const long long total = L * batch, total_j = total / R;
+    cudaError_t e;
+    const bool first = Ns == 1 && src;
     switch (R) {
-      case 16: pass_pow2_kernel<16><<<grid_for(total_j, num_sms), 256, 0, st>>>(x, y, tw, L, Ns, total_j); break;
-      case 8: pass_pow2_kernel<8><<<grid_for(total_j, num_sms), 256, 0, st>>>(x, y, tw, L, Ns, total_j); break;
-      case 4: pass_pow2_kernel<4><<<grid_for(total_j, num_sms), 256, 0, st>>>(x, y, tw, L, Ns, total_j); break;
-      case 2: pass_pow2_kernel<2><<<grid_for(total_j, num_sms), 256, 0, st>>>(x, y, tw, L, Ns, total_j); break;
-      default: pass_any_kernel<<<grid_for(total, num_sms), 256, 0, st>>>(x, y, tw, L, R, Ns, total); break;
+#define TGA_PASS(RR)                                                                          \
+  case RR:                                                                                    \
+    e = run_pass64<RR, false>(x, none, y, tw, L, batch, Ns, st);                              \
+    break;
+#define TGA_PASS2(RR)                                                                         \
+  case RR:                                                                                    \
+    e = first ? run_pass64<RR, true>(x, *src, y, tw, L, batch, Ns, st)                        \
+              : run_pass64<RR, false>(x, none, y, tw, L, batch, Ns, st);                      \
+    break;
+      TGA_PASS2(32) TGA_PASS2(16) TGA_PASS2(8) TGA_PASS2(4) TGA_PASS(2)
+      TGA_PASS(33) TGA_PASS(25) TGA_PASS(15) TGA_PASS(31) TGA_PASS(13) TGA_PASS(11) TGA_PASS(7) TGA_PASS(5) TGA_PASS(3)
+#undef TGA_PASS
+#undef TGA_PASS2
+      default: {
+        const long long total = L * batch;
+        pass_any_kernel<<<grid_for(total, num_sms), 256, 0, st>>>(x, y, tw, L, R, Ns, total);
+        e = cudaGetLastError();
+      }
     }
     kernel_launch_add(1);
-    if ((*err = cudaGetLastError()) != cudaSuccess) return x;
+    if (e != cudaSuccess) return e;
     Ns *= R;
     double2* t = x;
     x = y;
     y = t;
   }
-  return x;
+  *result = x;
+  return cudaSuccess;
 }
 
 // ---- Bluestein: X[k] = c[k] sum_m (x[m] c[m]) conj(c[k - m]), c[m] = W_{2L}^{m^2}
@@ -203,23 +396,63 @@ __global__ void postmul64_kernel(const double2* __restrict__ y, const double2* _
   }
 }
 
+// The rows' samples as doubles (Bluestein's input): +-1 - mean
+__global__ void samples64_kernel(FirstSource src, long long n, double* __restrict__ z) {
+  const uint8_t* row = src.bits + (size_t)blockIdx.y * src.row_bytes;
+  const double m = src.mean[blockIdx.y];
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const int bit = (__ldg(row + (i >> 3)) >> (7 - (int)(i & 7))) & 1;
+    z[(size_t)blockIdx.y * n + i] = (bit ? 1.0 : -1.0) - m;
+  }
+}
+
 // |X[k]|^2 for k < L of the real record whose n = 2 L point spectrum is
-// recovered from Z = FFT_L(z), z[m] = x[2m] + i x[2m+1]
-__global__ void real_power_kernel(const double2* __restrict__ Z, long long L, int batch, double* __restrict__ p) {
-  const long long total = L * batch;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long a = i / L, k = i - a * L;
-    const double2 zk = Z[a * L + k], zc = Z[a * L + (k == 0 ? 0 : L - k)];
+// recovered from Z = FFT_L(z), z[m] = x[2m] + i x[2m+1] (L even), and the
+// histogram of their top digits (first pass of the median's radix select).
+// A thread takes bins k and L - k, which need the same two values of Z and one
+// twiddle W_n^k = exp(-i pi k / L): the table's W_L^{k / 2}, times w1 = W_n for
+// an odd k, or sincospi where there is no table.  The histogram costs no pass
+// of its own over the powers.
+constexpr int kPowerIters = 16;
+__global__ void __launch_bounds__(256) real_power_kernel(const double2* __restrict__ Z, const double2* __restrict__ tw,
+                                                         double2 w1, unsigned L, double* __restrict__ p,
+                                                         unsigned* __restrict__ hist) {
+  __shared__ unsigned sh[kRfiDigits];
+  for (int i = threadIdx.x; i < kRfiDigits; i += 256) sh[i] = 0;
+  __syncthreads();
+  const double2* z = Z + (size_t)blockIdx.y * L;
+  double* row = p + (size_t)blockIdx.y * L;
+  auto put = [&](unsigned k, double v) {
+    row[k] = v;
+    atomicAdd(&sh[(unsigned)((unsigned long long)__double_as_longlong(v) >> kRfiShift0)], 1u);
+  };
+  for (int it = 0; it < kPowerIters; ++it) {
+    const unsigned k = (blockIdx.x * kPowerIters + it) * 256 + threadIdx.x;
+    if (k > L / 2) break;
+    const double2 zk = z[k], zc = z[k == 0 ? 0 : L - k];
     const double2 e = make_double2(0.5 * (zk.x + zc.x), 0.5 * (zk.y - zc.y));  // (Z[k] + conj Z[L-k]) / 2
     const double2 o = make_double2(0.5 * (zk.x - zc.x), 0.5 * (zk.y + zc.y));  // (Z[k] - conj Z[L-k]) / 2
-    double s, c;
-    sincospi((double)k / (double)L, &s, &c);  // W_n^k = exp(-i pi k / L) = (c, -s)
-    // X = e - i W o
-    const double2 wo = make_double2(c * o.x + s * o.y, c * o.y - s * o.x);
-    const double xr = e.x + wo.y, xi = e.y - wo.x;
-    p[i] = xr * xr + xi * xi;
+    double2 w;  // exp(-i pi k / L)
+    if (tw) {
+      w = __ldg(tw + k / 2);
+      if (k & 1u) w = cmul64(w, w1);
+    } else {
+      double s, c;
+      sincospi((double)k / (double)L, &s, &c);
+      w = make_double2(c, -s);
+    }
+    const double2 wo = cmul64(w, o);
+    // X[k] = e - i w o; X[L - k] = conj(e) - i conj(w o)
+    const double ar = e.x + wo.y, ai = e.y - wo.x;
+    put(k, ar * ar + ai * ai);
+    if (k != 0 && 2 * k != L) {
+      const double br = e.x - wo.y, bi = -e.y - wo.x;
+      put(L - k, br * br + bi * bi);
+    }
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kRfiDigits; i += 256)
+    if (sh[i]) atomicAdd(hist + (size_t)blockIdx.y * 2 * kRfiDigits + i, sh[i]);
 }
 
 long long next_pow2(long long v) {
@@ -238,59 +471,66 @@ size_t fft64_workspace_bytes(long long n, int batch) {
   return (size_t)(M + L + 3 * M) * 16;  // table of M, chirp, filter spectrum, two work buffers
 }
 
-cudaError_t real_power_spectrum(double* d_x, void* d_buf, void* d_work, long long n, int batch, double* d_p,
-                                int num_sms, cudaStream_t st, std::string* why) {
-  if (n % 2 != 0 || n < 4) {
-    *why = "the RFI spectrum needs an even record of at least 4 samples";
+cudaError_t real_power_spectrum(const uint8_t* d_bits, size_t row_bytes, const double* d_mean, double* d_x, void* d_buf,
+                                void* d_work, int batch, double* d_p, unsigned* d_hist, int num_sms, cudaStream_t st,
+                                std::string* why) {
+  const long long n = (long long)row_bytes * 8, L = n / 2;
+  if (n < 8 || L >= (1LL << 30) || batch > 65535) {
+    *why = "the RFI spectrum needs records of 8 samples up to 2^31 and at most 65535 antennas";
     return cudaErrorInvalidValue;
   }
-  const long long L = n / 2;
-  double2* z = reinterpret_cast<double2*>(d_x);  // the record as L complex points
+  double2* z = reinterpret_cast<double2*>(d_x);
   double2* buf = static_cast<double2*>(d_buf);
   double2* work = static_cast<double2*>(d_work);
+  const FirstSource src = {d_bits, row_bytes, d_mean};
   cudaError_t e = cudaSuccess;
   std::vector<int> radices;
   double2* Z = nullptr;
+  const double2* tw = nullptr;
   if (factorise(L, &radices)) {
+    // L is a multiple of 4, so the first radix is a power of two, at least 4
     twiddle64_kernel<<<grid_for(L, num_sms), 256, 0, st>>>(work, L);
     kernel_launch_add(1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    Z = stockham(z, buf, work, L, batch, radices, num_sms, st, &e);
-    if (e != cudaSuccess) return e;
+    tw = work;
+    if ((e = stockham(z, buf, &src, work, L, batch, radices, num_sms, st, &Z)) != cudaSuccess) return e;
   } else {
     // Bluestein per sequence: convolution length M = 2^m >= 2L - 1
     const long long M = next_pow2(2 * L - 1);
     factorise(M, &radices);
-    double2* tw = work;
-    double2* chirp = tw + M;
+    double2* twM = work;
+    double2* chirp = twM + M;
     double2* H = chirp + L;
     double2* u = H + M;
     double2* v = u + M;
-    twiddle64_kernel<<<grid_for(M, num_sms), 256, 0, st>>>(tw, M);
+    samples64_kernel<<<dim3(256, (unsigned)batch), 256, 0, st>>>(src, n, d_x);
+    twiddle64_kernel<<<grid_for(M, num_sms), 256, 0, st>>>(twM, M);
     chirp64_kernel<<<grid_for(L, num_sms), 256, 0, st>>>(chirp, L);
     chirp_filter64_kernel<<<grid_for(M, num_sms), 256, 0, st>>>(chirp, L, M, u);
-    kernel_launch_add(3);
+    kernel_launch_add(4);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    double2* h = stockham(u, v, tw, M, 1, radices, num_sms, st, &e);
-    if (e != cudaSuccess) return e;
+    double2* h = nullptr;
+    if ((e = stockham(u, v, nullptr, twM, M, 1, radices, num_sms, st, &h)) != cudaSuccess) return e;
     if (h != H) e = cudaMemcpyAsync(H, h, (size_t)M * 16, cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) return e;
     for (int a = 0; a < batch; ++a) {
       premul64_kernel<<<grid_for(M, num_sms), 256, 0, st>>>(z + a * L, chirp, L, M, u);
       kernel_launch_add(1);
-      double2* y = stockham(u, v, tw, M, 1, radices, num_sms, st, &e);
-      if (e != cudaSuccess) return e;
+      double2 *y = nullptr, *w = nullptr;
+      if ((e = stockham(u, v, nullptr, twM, M, 1, radices, num_sms, st, &y)) != cudaSuccess) return e;
       conjmul64_kernel<<<grid_for(M, num_sms), 256, 0, st>>>(y, H, M);
       kernel_launch_add(1);
-      double2* w = stockham(y, y == u ? v : u, tw, M, 1, radices, num_sms, st, &e);
-      if (e != cudaSuccess) return e;
+      if ((e = stockham(y, y == u ? v : u, nullptr, twM, M, 1, radices, num_sms, st, &w)) != cudaSuccess) return e;
       postmul64_kernel<<<grid_for(L, num_sms), 256, 0, st>>>(w, chirp, L, M, buf + a * L);
       kernel_launch_add(1);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     Z = buf;
   }
-  real_power_kernel<<<grid_for(L * batch, num_sms), 256, 0, st>>>(Z, L, batch, d_p);
+  const double half_step = 3.14159265358979323846 / (double)L;
+  const unsigned blocks = (unsigned)((L / 2 + 1 + 256 * kPowerIters - 1) / (256 * kPowerIters));
+  real_power_kernel<<<dim3(blocks, (unsigned)batch), 256, 0, st>>>(
+      Z, tw, make_double2(std::cos(half_step), -std::sin(half_step)), (unsigned)L, d_p, d_hist);
   kernel_launch_add(1);
   return cudaGetLastError();
 }

@@ -6,7 +6,10 @@
 //     the first n/2 bins), with this library's own f64 FFT (fft64.cu) over
 //     all antennas at once;
 //   * the median bin power, exactly: a radix select over the bit patterns of
-//     the non-negative powers (8 passes of 8 bits), no sorting;
+//     the non-negative powers (RfiBufs), no sorting.  24 rows of 818400 bins: the
+//     eight histogram passes and their serial digit searches took 0.41 ms;
+//     the first digit is counted where the powers are made, the second and the
+//     gathering of the few bins left are a pass each, 0.08 ms in all;
 //   * local maxima p[k] > p[k-1], p[k] >= p[k+1] with 10 log10(p / floor) >
 //     15 dB (rfi.rs:113-123), appended to a per-antenna list that the host
 //     clusters (10 kHz, strongest first, at most 3 lines; rfi.rs:125-139);
@@ -15,9 +18,9 @@
 //     + (n - L) m^2 with sum s s' = (n - L) - 2 popcount(b_i xor b_{i+L}).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <string>
-#include <vector>
 
 #include "engine.h"
 
@@ -25,56 +28,138 @@ namespace tga {
 
 namespace {
 
-__global__ void rfi_prepare_kernel(const uint8_t* __restrict__ bits, size_t row_bytes, const double* __restrict__ mean,
-                                   long long n, double* __restrict__ z) {
-  const int a = blockIdx.y;
-  const uint8_t* row = bits + (size_t)a * row_bytes;
-  const double m = mean[a];
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int bit = (__ldg(row + (i >> 3)) >> (7 - (int)(i & 7))) & 1;
-    z[(size_t)a * n + i] = (bit ? 1.0 : -1.0) - m;
+// the digit holding rank[a] among kRfiDigits counts, one block per antenna:
+// narrows the prefix and the rank
+__global__ void __launch_bounds__(256) rfi_select_kernel(const unsigned* __restrict__ hist, int digit, int shift,
+                                                         unsigned rank0, unsigned long long* __restrict__ prefix,
+                                                         unsigned* __restrict__ rank) {
+  __shared__ unsigned part[256];
+  constexpr int PER = kRfiDigits / 256;
+  const int a = blockIdx.x, t = threadIdx.x;
+  const unsigned* h = hist + ((size_t)a * 2 + digit) * kRfiDigits + t * PER;
+  unsigned sum = 0;
+  for (int i = 0; i < PER; ++i) sum += h[i];
+  part[t] = sum;
+  __syncthreads();
+  for (int o = 1; o < 256; o <<= 1) {  // inclusive scan
+    const unsigned v = t >= o ? part[t - o] : 0u;
+    __syncthreads();
+    part[t] += v;
+    __syncthreads();
+  }
+  const unsigned r = digit == 0 ? rank0 : rank[a];
+  unsigned cum = part[t] - sum;
+  __syncthreads();
+  if (r >= cum && r < cum + sum) {
+    int d = 0;
+    while (cum + h[d] <= r) cum += h[d++];
+    prefix[a] = (digit == 0 ? 0ull : prefix[a]) | ((unsigned long long)(t * PER + d) << shift);
+    rank[a] = r - cum;
   }
 }
 
-// one radix-select pass: histogram of the 8-bit digit at `shift` over the
-// elements whose higher digits equal the prefix found so far
-__global__ void rfi_hist_kernel(const double* __restrict__ p, long long half, int shift,
-                                const unsigned long long* __restrict__ prefix, unsigned* __restrict__ hist) {
-  __shared__ unsigned sh[256];
-  const int a = blockIdx.y;
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) sh[i] = 0;
-  __syncthreads();
-  const unsigned long long mask = shift >= 56 ? 0ull : (~0ull << (shift + 8));
-  const unsigned long long pre = prefix[a] & mask;
-  const double* row = p + (size_t)a * half;
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < half; k += (long long)gridDim.x * blockDim.x) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(row[k]);
-    if ((u & mask) == pre) atomicAdd(&sh[(u >> shift) & 255u], 1u);
+// f(bits) for every power of antenna a's row (an even number of them, rows
+// 16-byte aligned): four 16-byte loads in flight per thread
+template <class F>
+__device__ __forceinline__ void for_powers(const double* __restrict__ p, unsigned half, int a, F&& f) {
+  const double2* row = reinterpret_cast<const double2*>(p + (size_t)a * half);
+  const unsigned n = half / 2, stride = gridDim.x * 256;
+  for (unsigned k = blockIdx.x * 256 + threadIdx.x; k < n; k += 4 * stride) {
+    double2 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (k + i * stride < n) v[i] = __ldg(row + k + i * stride);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (k + i * stride < n) {
+        f((unsigned long long)__double_as_longlong(v[i].x));
+        f((unsigned long long)__double_as_longlong(v[i].y));
+      }
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 256; i += blockDim.x)
-    if (sh[i]) atomicAdd(&hist[(size_t)a * 256 + i], sh[i]);
 }
 
-// picks the digit holding rank[a], narrows the prefix and the rank, clears
-// the histogram for the next pass (one thread per antenna)
-__global__ void rfi_select_kernel(int n_ant, int shift, unsigned* __restrict__ hist,
-                                  unsigned long long* __restrict__ prefix, unsigned long long* __restrict__ rank) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= n_ant) return;
-  unsigned* h = hist + (size_t)a * 256;
-  unsigned long long r = rank[a], cum = 0;
-  int d = 255;
-  for (int i = 0; i < 256; ++i) {
-    if (cum + h[i] > r) {
-      d = i;
-      break;
+// histogram of the second digit over the bins whose first digit is the prefix's
+__global__ void __launch_bounds__(256) rfi_hist_kernel(const double* __restrict__ p, unsigned half,
+                                                       const unsigned long long* __restrict__ prefix,
+                                                       unsigned* __restrict__ hist) {
+  __shared__ unsigned sh[kRfiDigits];
+  const int a = blockIdx.y;
+  for (int i = threadIdx.x; i < kRfiDigits; i += 256) sh[i] = 0;
+  __syncthreads();
+  const unsigned long long pre = prefix[a] >> kRfiShift0;
+  for_powers(p, half, a, [&](unsigned long long u) {
+    if (u >> kRfiShift0 == pre) atomicAdd(&sh[(u >> kRfiShift1) & (kRfiDigits - 1)], 1u);
+  });
+  __syncthreads();
+  for (int i = threadIdx.x; i < kRfiDigits; i += 256)
+    if (sh[i]) atomicAdd(hist + ((size_t)a * 2 + 1) * kRfiDigits + i, sh[i]);
+}
+
+// the bins that share both digits, and their number (it may exceed the list)
+__global__ void __launch_bounds__(256) rfi_gather_kernel(const double* __restrict__ p, unsigned half,
+                                                         const unsigned long long* __restrict__ prefix,
+                                                         unsigned* __restrict__ n_list,
+                                                         unsigned long long* __restrict__ list) {
+  const int a = blockIdx.y;
+  const unsigned long long pre = prefix[a] >> kRfiShift1;
+  for_powers(p, half, a, [&](unsigned long long u) {
+    if (u >> kRfiShift1 == pre) {
+      const unsigned i = atomicAdd(n_list + a, 1u);
+      if (i < (unsigned)kRfiList) list[(size_t)a * kRfiList + i] = u;
     }
-    cum += h[i];
+  });
+}
+
+// the element of rank[a] among the gathered bins, one block per antenna.  More
+// bins than the list holds (many equal powers): three more digits over the
+// whole row by this block.
+__global__ void __launch_bounds__(256) rfi_median_kernel(const double* __restrict__ p, unsigned half,
+                                                         const unsigned* __restrict__ n_list,
+                                                         const unsigned long long* __restrict__ list,
+                                                         const unsigned* __restrict__ rank,
+                                                         unsigned long long* __restrict__ prefix) {
+  __shared__ unsigned sh[kRfiDigits];
+  __shared__ unsigned long long s_pre;
+  __shared__ unsigned s_rank;
+  const int a = blockIdx.x;
+  const unsigned n = n_list[a], r = rank[a];
+  if (n <= (unsigned)kRfiList) {
+    const unsigned long long* l = list + (size_t)a * kRfiList;
+    for (unsigned i = threadIdx.x; i < n; i += 256) {
+      unsigned less = 0, same = 0;
+      for (unsigned k = 0; k < n; ++k) {
+        less += l[k] < l[i] ? 1u : 0u;
+        same += l[k] == l[i] ? 1u : 0u;
+      }
+      if (r >= less && r < less + same) prefix[a] = l[i];  // equal elements write the same value
+    }
+    return;
   }
-  for (int i = 0; i < 256; ++i) h[i] = 0;
-  prefix[a] |= (unsigned long long)d << shift;
-  rank[a] = r - cum;
+  if (threadIdx.x == 0) {
+    s_pre = prefix[a];
+    s_rank = r;
+  }
+  const double* row = p + (size_t)a * half;
+  for (int shift = kRfiShift1 - 13; shift > -13; shift -= 13) {
+    const int lo = shift < 0 ? 0 : shift, width = shift < 0 ? 13 + shift : 13;
+    for (int i = threadIdx.x; i < kRfiDigits; i += 256) sh[i] = 0;
+    __syncthreads();
+    const unsigned long long pre = s_pre >> (lo + width);
+    for (unsigned k = threadIdx.x; k < half; k += 256) {
+      const unsigned long long u = (unsigned long long)__double_as_longlong(__ldg(row + k));
+      if (u >> (lo + width) == pre) atomicAdd(&sh[(u >> lo) & ((1u << width) - 1)], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned left = s_rank;
+      int d = 0;
+      while (sh[d] <= left) left -= sh[d++];
+      s_rank = left;
+      s_pre |= (unsigned long long)d << lo;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) prefix[a] = s_pre;
 }
 
 __global__ void rfi_peaks_kernel(const double* __restrict__ p, long long half, const unsigned long long* __restrict__ floor_bits,
@@ -86,7 +171,8 @@ __global__ void rfi_peaks_kernel(const double* __restrict__ p, long long half, c
   for (long long k = 1 + (long long)blockIdx.x * blockDim.x + threadIdx.x; k < half - 1;
        k += (long long)gridDim.x * blockDim.x) {
     const double v = row[k];
-    if (v > row[k - 1] && v >= row[k + 1]) {
+    // (15 dB is a factor of 31.62: the logarithm is taken only where it can matter)
+    if (v > row[k - 1] && v >= row[k + 1] && v >= 31.6 * fl) {
       const double ex = 10.0 * log10(v / fl);
       if (ex > min_excess_db) {
         const unsigned idx = atomicAdd(&count[a], 1u);
@@ -143,43 +229,31 @@ __global__ void rfi_acf_kernel(const uint8_t* __restrict__ bits, size_t row_byte
 
 }  // namespace
 
-cudaError_t rfi_scan_device(const uint8_t* d_bits, int n_ant, size_t row_bytes, const double* d_mean, double* d_z,
-                            void* d_X, void* d_work, double* d_p, unsigned* d_hist, unsigned long long* d_prefix,
-                            unsigned long long* d_rank, int cap, unsigned* d_count, long long* d_bins,
-                            double* d_excess, unsigned long long* d_acf, int num_sms, cudaStream_t st,
-                            std::string* why) {
+cudaError_t rfi_scan_device(const uint8_t* d_bits, int n_ant, size_t row_bytes, const double* d_mean, const RfiBufs& b,
+                            int cap, int num_sms, cudaStream_t st, std::string* why) {
   const long long n = (long long)row_bytes * 8, half = n / 2;
   if (n_ant <= 0 || n < 8) return cudaSuccess;
   cudaError_t e;
-  dim3 g1(256, n_ant);
-  rfi_prepare_kernel<<<g1, 256, 0, st>>>(d_bits, row_bytes, d_mean, n, d_z);
-  kernel_launch_add(1);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  const size_t A = (size_t)n_ant;
+  if ((e = cudaMemsetAsync(b.hist, 0, A * 2 * kRfiDigits * sizeof(unsigned), st)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(b.n_list, 0, A * sizeof(unsigned), st)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(b.count, 0, A * sizeof(unsigned), st)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(b.acf, 0, A * 9 * sizeof(unsigned long long), st)) != cudaSuccess) return e;
   // powers of the first n/2 bins of every antenna's f64 spectrum
-  if ((e = real_power_spectrum(d_z, d_X, d_work, n, n_ant, d_p, num_sms, st, why)) != cudaSuccess) return e;
+  e = real_power_spectrum(d_bits, row_bytes, d_mean, b.z, b.X, b.work, n_ant, b.p, b.hist, num_sms, st, why);
+  if (e != cudaSuccess) return e;
   // median bin power: rank half / 2 (rfi.rs:110-111)
-  if ((e = cudaMemsetAsync(d_hist, 0, (size_t)n_ant * 256 * sizeof(unsigned), st)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(d_prefix, 0, (size_t)n_ant * sizeof(unsigned long long), st)) != cudaSuccess) return e;
-  {
-    const unsigned long long r = (unsigned long long)(half / 2);
-    std::vector<unsigned long long> rk((size_t)n_ant, r);
-    if ((e = cudaMemcpyAsync(d_rank, rk.data(), rk.size() * sizeof(r), cudaMemcpyHostToDevice, st)) != cudaSuccess)
-      return e;
-    for (int shift = 56; shift >= 0; shift -= 8) {
-      rfi_hist_kernel<<<g1, 256, 0, st>>>(d_p, half, shift, d_prefix, d_hist);
-      rfi_select_kernel<<<(n_ant + 63) / 64, 64, 0, st>>>(n_ant, shift, d_hist, d_prefix, d_rank);
-      kernel_launch_add(2);
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;  // rk is a host temporary
-  }
-  if ((e = cudaMemsetAsync(d_count, 0, (size_t)n_ant * sizeof(unsigned), st)) != cudaSuccess) return e;
-  rfi_peaks_kernel<<<g1, 256, 0, st>>>(d_p, half, d_prefix, 15.0, cap, d_count, d_bins, d_excess);
-  kernel_launch_add(1);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(d_acf, 0, (size_t)n_ant * 9 * sizeof(unsigned long long), st)) != cudaSuccess) return e;
-  rfi_acf_kernel<<<dim3(64, n_ant), 256, 0, st>>>(d_bits, row_bytes, n, d_acf);
-  kernel_launch_add(1);
+  const unsigned h = (unsigned)half;
+  const dim3 g((unsigned)std::min<long long>(std::max(32, 8 * num_sms / n_ant), (half + 2047) / 2048), (unsigned)n_ant);
+  rfi_select_kernel<<<n_ant, 256, 0, st>>>(b.hist, 0, kRfiShift0, h / 2, b.prefix, b.rank);
+  rfi_hist_kernel<<<g, 256, 0, st>>>(b.p, h, b.prefix, b.hist);
+  rfi_select_kernel<<<n_ant, 256, 0, st>>>(b.hist, 1, kRfiShift1, 0u, b.prefix, b.rank);
+  rfi_gather_kernel<<<g, 256, 0, st>>>(b.p, h, b.prefix, b.n_list, b.list);
+  rfi_median_kernel<<<n_ant, 256, 0, st>>>(b.p, h, b.n_list, b.list, b.rank, b.prefix);
+  rfi_peaks_kernel<<<dim3(256, (unsigned)n_ant), 256, 0, st>>>(b.p, half, b.prefix, 15.0, cap, b.count, b.bins,
+                                                               b.excess);
+  rfi_acf_kernel<<<dim3(64, (unsigned)n_ant), 256, 0, st>>>(d_bits, row_bytes, n, b.acf);
+  kernel_launch_add(7);
   return cudaGetLastError();
 }
 

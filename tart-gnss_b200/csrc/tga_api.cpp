@@ -1836,31 +1836,44 @@ int tga_rfi_scan(tga_ctx* ctx, const uint8_t* h_bits, size_t n_ant, size_t row_b
     ctx->h2d += A * row_bytes;
     double* d_mean = (double*)ctx->buf("rfi.mean", A * sizeof(double));
     CK(launch_antenna_means(d_bits, (int)A, row_bytes, d_mean, st));
-    double* d_z = (double*)ctx->buf("rfi.z", A * (size_t)n * sizeof(double));
-    void* d_X = ctx->buf("rfi.X", A * (size_t)(n / 2 + 1) * 16);
-    void* d_work = ctx->buf("rfi.work", fft64_workspace_bytes(n, (int)A));
-    double* d_p = (double*)ctx->buf("rfi.p", A * (size_t)half * sizeof(double));
-    unsigned* d_hist = (unsigned*)ctx->buf("rfi.hist", A * 256 * sizeof(unsigned));
-    unsigned long long* d_prefix = (unsigned long long*)ctx->buf("rfi.prefix", A * 8);
-    unsigned long long* d_rank = (unsigned long long*)ctx->buf("rfi.rank", A * 8);
-    unsigned* d_count = (unsigned*)ctx->buf("rfi.count", A * sizeof(unsigned));
-    long long* d_bins = (long long*)ctx->buf("rfi.bins", A * kCap * sizeof(long long));
-    double* d_excess = (double*)ctx->buf("rfi.excess", A * kCap * sizeof(double));
-    unsigned long long* d_acf = (unsigned long long*)ctx->buf("rfi.acf", A * 9 * 8);
+    RfiBufs rb;
+    rb.z = (double*)ctx->buf("rfi.z", A * (size_t)n * sizeof(double));
+    rb.X = ctx->buf("rfi.X", A * (size_t)(n / 2 + 1) * 16);
+    rb.work = ctx->buf("rfi.work", fft64_workspace_bytes(n, (int)A));
+    rb.p = (double*)ctx->buf("rfi.p", A * (size_t)half * sizeof(double));
+    rb.hist = (unsigned*)ctx->buf("rfi.hist", A * 2 * kRfiDigits * sizeof(unsigned));
+    rb.prefix = (unsigned long long*)ctx->buf("rfi.prefix", A * 8);
+    rb.rank = (unsigned*)ctx->buf("rfi.rank", A * sizeof(unsigned));
+    rb.n_list = (unsigned*)ctx->buf("rfi.n_list", A * sizeof(unsigned));
+    rb.list = (unsigned long long*)ctx->buf("rfi.list", A * kRfiList * 8);
+    rb.count = (unsigned*)ctx->buf("rfi.count", A * sizeof(unsigned));
+    rb.bins = (long long*)ctx->buf("rfi.bins", A * kCap * sizeof(long long));
+    rb.excess = (double*)ctx->buf("rfi.excess", A * kCap * sizeof(double));
+    rb.acf = (unsigned long long*)ctx->buf("rfi.acf", A * 9 * 8);
     std::string why;
-    const cudaError_t e = rfi_scan_device(d_bits, (int)A, row_bytes, d_mean, d_z, d_X, d_work, d_p, d_hist, d_prefix,
-                                          d_rank, kCap, d_count, d_bins, d_excess, d_acf, ctx->num_sms, st, &why);
+    const cudaError_t e = rfi_scan_device(d_bits, (int)A, row_bytes, d_mean, rb, kCap, ctx->num_sms, st, &why);
     if (!why.empty()) throw std::runtime_error(why);
     CK(e);
     std::vector<double> mean(A);
     std::vector<unsigned> count(A);
     std::vector<unsigned long long> acf(A * 9);
     CK(cudaMemcpyAsync(mean.data(), d_mean, A * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(count.data(), d_count, A * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(acf.data(), d_acf, A * 9 * 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(count.data(), rb.count, A * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(acf.data(), rb.acf, A * 9 * 8, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    for (size_t a = 0; a < A; ++a)
+    unsigned most = 0;
+    for (size_t a = 0; a < A; ++a) {
       if (count[a] > (unsigned)kCap) throw std::runtime_error("more than 65536 candidate RFI lines on one antenna");
+      most = std::max(most, count[a]);
+    }
+    // the candidate lists of all antennas in one copy each
+    std::vector<long long> all_bins(A * most);
+    std::vector<double> all_ex(A * most);
+    if (most) {
+      CK(cudaMemcpy2DAsync(all_bins.data(), most * 8, rb.bins, (size_t)kCap * 8, most * 8, A, cudaMemcpyDeviceToHost, st));
+      CK(cudaMemcpy2DAsync(all_ex.data(), most * 8, rb.excess, (size_t)kCap * 8, most * 8, A, cudaMemcpyDeviceToHost, st));
+      CK(cudaStreamSynchronize(st));
+    }
     const int lags[3] = {1, 3, 16};
     for (size_t a = 0; a < A; ++a) {
       tga_rfi_channel& ch = out[a];
@@ -1887,12 +1900,8 @@ int tga_rfi_scan(tga_ctx* ctx, const uint8_t* h_bits, size_t n_ant, size_t row_b
       // candidate lines: strongest first, ties in bin order (a stable sort of
       // the bin-ordered list, rfi.rs:126), then 10 kHz clustering
       const unsigned c = count[a];
-      std::vector<long long> bins(c);
-      std::vector<double> ex(c);
-      if (c) {
-        CK(cudaMemcpy(bins.data(), d_bins + a * kCap, c * sizeof(long long), cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(ex.data(), d_excess + a * kCap, c * sizeof(double), cudaMemcpyDeviceToHost));
-      }
+      const long long* bins = all_bins.data() + a * most;
+      const double* ex = all_ex.data() + a * most;
       std::vector<size_t> idx(c);
       for (size_t i = 0; i < c; ++i) idx[i] = i;
       std::sort(idx.begin(), idx.end(), [&](size_t x, size_t y) {
