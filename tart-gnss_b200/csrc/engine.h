@@ -53,6 +53,14 @@ struct FineTask {
   long long start, length;
 };
 
+// A frequency scan: R of the task at n_k frequencies, number k0 of them the
+// task's own, df_over_fs apart; point k lands in out[task.slot + k].
+struct FineScan {
+  FineTask task;
+  int n_k, k0;
+  double df_over_fs;
+};
+
 struct SearchDims {
   int n_ant = 0, nb = 0, n_prn = 0;
   const double* fc = nullptr;  // device Doppler grid [nb]
@@ -176,6 +184,13 @@ cudaError_t launch_bits_to_signal(const uint8_t* d_bits, size_t row_bytes, int r
 cudaError_t launch_fine_sums(const uint8_t* d_bits, int n_ant, size_t row_bytes, const double* d_mean,
                              const FineTask* d_tasks, int n_tasks, long long max_length, double* d_out,
                              cudaStream_t st);
+
+// the first of those sums alone, R, at the frequencies of n_tasks scans
+// (n_points in all, at most max_k each): out[point][antenna][2], zeroed and
+// accumulated
+cudaError_t launch_fine_scan(const uint8_t* d_bits, int n_ant, size_t row_bytes, const double* d_mean,
+                             const FineScan* d_tasks, int n_tasks, int n_points, int max_k, long long max_length,
+                             double* d_out, cudaStream_t st);
 
 // narrowband RFI scan of every antenna row (rfi.rs:91-168): f64 spectrum,
 // exact median bin power, local maxima above 15 dB (up to cap per antenna,

@@ -1571,6 +1571,29 @@ void fine_sums(tga_ctx* ctx, const uint8_t* d_bits, size_t A, size_t row_bytes, 
   }
 }
 
+// R of every point of the scans, normalised by the window length: out[point][antenna]
+void fine_scan(tga_ctx* ctx, const uint8_t* d_bits, size_t A, size_t row_bytes, const double* d_mean,
+               const std::vector<FineScan>& scans, size_t points, std::vector<cplx>& out) {
+  FineScan* d_scans = (FineScan*)ctx->buf("fine.scans", scans.size() * sizeof(FineScan));
+  double* d_out = (double*)ctx->buf("fine.scan_sums", points * A * 2 * sizeof(double));
+  CK(cudaMemcpyAsync(d_scans, scans.data(), scans.size() * sizeof(FineScan), cudaMemcpyHostToDevice, ctx->stream));
+  long long max_len = 0;
+  int max_k = 0;
+  for (const FineScan& q : scans) {
+    max_len = std::max(max_len, q.task.length);
+    max_k = std::max(max_k, q.n_k);
+  }
+  CK(launch_fine_scan(d_bits, (int)A, row_bytes, d_mean, d_scans, (int)scans.size(), (int)points, max_k, max_len, d_out,
+                      ctx->stream));
+  out.resize(points * A);
+  CK(cudaMemcpyAsync(out.data(), d_out, out.size() * sizeof(cplx), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  for (const FineScan& q : scans) {
+    const double inv = 1.0 / (double)q.task.length;
+    for (size_t i = (size_t)q.task.slot * A; i < ((size_t)q.task.slot + q.n_k) * A; ++i) out[i] *= inv;
+  }
+}
+
 // P = |sum_a exp(-i phi_a) R_a|^2 with its gradient and Hessian in the order
 // (tau, f, phi_0 .. phi_{A-1}); g and H may be null
 void fine_assemble(const cplx* R, int A, const double* phi, double* P, double* g, double* H) {
@@ -1700,25 +1723,33 @@ int tga_fine_acquire(tga_ctx* ctx, const uint8_t* h_bits, size_t n_ant, size_t r
     //    main lobe of a long window, so the start may sit on a side lobe
     std::vector<int> nscan(n_tasks, 0);
     std::vector<FineTask> batch;
+    std::vector<FineScan> scans;
+    size_t points = 0;
     for (size_t i = 0; i < n_tasks; ++i) {
       const double win = (double)tasks[i].length / fs;
       const double df = 0.25 / win;
       const double hw = o.scan_hw == 0.0 ? 150.0 + 1.0 / win : o.scan_hw;
       const int K = hw < 0 ? 0 : (int)std::ceil(hw / df);
       nscan[i] = K;
-      for (int k = -K; k <= K; ++k)
-        batch.push_back(fine_task(jobs[i], fs, tasks[i].code_phase, tasks[i].frequency + k * df, (int)batch.size()));
+      FineScan sc;
+      sc.task = fine_task(jobs[i], fs, tasks[i].code_phase, tasks[i].frequency, (int)points);
+      sc.n_k = 2 * K + 1;
+      sc.k0 = K;
+      sc.df_over_fs = df / fs;
+      points += (size_t)sc.n_k;
+      scans.push_back(sc);
     }
-    fine_sums(ctx, d_bits, n_ant, row_bytes, d_mean, batch, R);
+    fine_scan(ctx, d_bits, n_ant, row_bytes, d_mean, scans, points, R);
     size_t pos = 0;
     for (size_t i = 0; i < n_tasks; ++i) {
       const double df = 0.25 * fs / (double)tasks[i].length;
       const int K = nscan[i];
       double best = -1;
       int kb = 0;
-      std::vector<double> tmp;
       for (int k = -K; k <= K; ++k, ++pos) {
-        const double p = aligned(&R[pos * n_ant * 6], tmp);
+        double s = 0;
+        for (int a = 0; a < A; ++a) s += std::abs(R[pos * n_ant + a]);
+        const double p = s * s;  // P with every antenna phase-aligned
         if (k == 0) out[i].power_start = p;
         if (p > best) {
           best = p;
