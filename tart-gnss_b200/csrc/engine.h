@@ -164,15 +164,23 @@ cudaError_t launch_acr_batch(const double* d_ra, int n, int table, double* d_cn0
 cudaError_t launch_xcorr_matrix(const uint8_t* d_bits, int n_ant, size_t row_bytes,
                                 unsigned long long* d_counts, cudaStream_t st);
 
-// Generic path (any length N): reference algorithm with Bluestein FFTs.
+// Generic path (any length N): the reference algorithm with FFTs of length N.
 struct GenericPlan {
   int N = 0;        // signal length
-  int Mpow2 = 0;    // Bluestein length (power of two >= 2N-1)
-  int log2M = 0;
+  int Mpow2 = 0;    // Bluestein length (power of two >= 2N-1) where N needs one
+};
+// The code replica: sample n is (sub)chip floor(n / spc) mod len, of chips[] or
+// (boc) of [+c0, -c0, +c1, -c1, ...]; the second hypothesis changes its sign
+// from sample `split` on.
+struct GenericCode {
+  const int8_t* chips = nullptr;
+  int len = 0;
+  bool boc = false;
+  double spc = 0.0;
+  int split = 0;
 };
 cudaError_t launch_generic(const GenericPlan& gp, const float* d_sig, const double* d_pp,
-                           const double* d_fc, int nb, const float* d_code_a,
-                           const float* d_code_b, int period, double fs, float2* d_work,
+                           const double* d_fc, int nb, const GenericCode& code, int period, double fs, float2* d_work,
                            size_t work_elems, float* d_corr, int* d_result_i, float* d_result_f,
                            cudaStream_t st);
 size_t generic_work_elems(const GenericPlan& gp, int nb);

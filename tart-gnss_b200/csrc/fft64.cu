@@ -32,8 +32,8 @@
 #include <string>
 #include <vector>
 
-#include "dft64_consts.cuh"
 #include "engine.h"
+#include "mixed_radix.cuh"
 
 namespace tga {
 
@@ -41,121 +41,12 @@ namespace {
 
 constexpr int kMaxRadix = 1024;
 
-__device__ __forceinline__ double2 cmul64(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
 // tw[m] = exp(-2 pi i m / L), m < L
 __global__ void twiddle64_kernel(double2* __restrict__ tw, long long L) {
   for (long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x; m < L; m += (long long)gridDim.x * blockDim.x) {
     double s, c;
     sincospi(2.0 * (double)m / (double)L, &s, &c);
     tw[m] = make_double2(c, -s);
-  }
-}
-
-template <int R> __device__ __forceinline__ double kcosd(int m);
-template <int R> __device__ __forceinline__ double ksind(int m);
-#define TGA_D64(R)                                                                        \
-  template <> __device__ __forceinline__ double kcosd<R>(int m) { return kCosD##R[m]; } \
-  template <> __device__ __forceinline__ double ksind<R>(int m) { return kSinD##R[m]; }
-TGA_D64(3)
-TGA_D64(5)
-TGA_D64(7)
-TGA_D64(11)
-TGA_D64(13)
-TGA_D64(25)
-TGA_D64(31)
-TGA_D64(32)
-#undef TGA_D64
-
-// Forward DFTs of register arrays, outputs streamed to st(k, value).
-// Odd prime R: pairs s_n = x_n + x_{R-n}, d_n = x_n - x_{R-n} halve the terms.
-template <int R, class St>
-__device__ __forceinline__ void dft64_prime(const double2 (&x)[R], St&& st) {
-  constexpr int H = (R - 1) / 2;
-  double2 s[H], d[H];
-#pragma unroll
-  for (int n = 1; n <= H; ++n) {
-    s[n - 1] = make_double2(x[n].x + x[R - n].x, x[n].y + x[R - n].y);
-    d[n - 1] = make_double2(x[n].x - x[R - n].x, x[n].y - x[R - n].y);
-  }
-  double2 X0 = x[0];
-#pragma unroll
-  for (int n = 0; n < H; ++n) X0 = make_double2(X0.x + s[n].x, X0.y + s[n].y);
-  const double2 x0 = x[0];
-  st(0, X0);
-#pragma unroll
-  for (int k = 1; k <= H; ++k) {
-    double2 A = x0, B = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int n = 1; n <= H; ++n) {
-      const double c = kcosd<R>((n * k) % R), sn = ksind<R>((n * k) % R);
-      A.x = fma(s[n - 1].x, c, A.x);
-      A.y = fma(s[n - 1].y, c, A.y);
-      B.x = fma(d[n - 1].x, sn, B.x);
-      B.y = fma(d[n - 1].y, sn, B.y);
-    }
-    st(k, make_double2(A.x + B.y, A.y - B.x));      // A - i B
-    st(R - k, make_double2(A.x - B.y, A.y + B.x));  // A + i B
-  }
-}
-
-// N a power of two up to 32: decimation in time over x[off + i stride]
-template <int N, int STRIDE, int M>
-__device__ __forceinline__ void dft64_pow2(const double2 (&x)[M], int off, double2 (&y)[N]) {
-  if constexpr (N == 1) {
-    y[0] = x[off];
-  } else {
-    double2 e[N / 2], o[N / 2];
-    dft64_pow2<N / 2, 2 * STRIDE>(x, off, e);
-    dft64_pow2<N / 2, 2 * STRIDE>(x, off + STRIDE, o);
-#pragma unroll
-    for (int k = 0; k < N / 2; ++k) {
-      double2 t = o[k];
-      if (4 * k == N)
-        t = make_double2(o[k].y, -o[k].x);  // times -i
-      else if (k > 0)
-        t = cmul64(o[k], make_double2(kcosd<32>(k * (32 / N)), -ksind<32>(k * (32 / N))));
-      y[k] = make_double2(e[k].x + t.x, e[k].y + t.y);
-      y[k + N / 2] = make_double2(e[k].x - t.x, e[k].y - t.y);
-    }
-  }
-}
-
-template <int R, class St>
-__device__ __forceinline__ void dft64(const double2 (&x)[R], St&& st) {
-  if constexpr ((R & (R - 1)) == 0) {
-    double2 y[R];
-    dft64_pow2<R, 1>(x, 0, y);
-#pragma unroll
-    for (int k = 0; k < R; ++k) st(k, y[k]);
-  } else if constexpr (R == 33 || R == 15) {
-    // 3 x P, coprime: n = (P n1 + 3 n2) mod R, k = (P (P^-1 mod 3) k1 + 3 (3^-1 mod P) k2) mod R
-    constexpr int P = R / 3, E1 = P * (P % 3 == 1 ? 1 : 2), E2 = 3 * (P == 11 ? 4 : 2);
-    double2 u[3][P];
-#pragma unroll
-    for (int n2 = 0; n2 < P; ++n2) {
-      const double2 t[3] = {x[(3 * n2) % R], x[(P + 3 * n2) % R], x[(2 * P + 3 * n2) % R]};
-      dft64_prime<3>(t, [&](int k1, double2 v) { u[k1][n2] = v; });
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < 3; ++k1)
-      dft64_prime<P>(u[k1], [&](int k2, double2 v) { st((E1 * k1 + E2 * k2) % R, v); });
-  } else if constexpr (R == 25) {
-    // n = 5 n1 + n2, k = k1 + 5 k2, twiddles W_25^{n2 k1}
-    double2 u[5][5];  // [k1][n2]
-#pragma unroll
-    for (int n2 = 0; n2 < 5; ++n2) {
-      const double2 t[5] = {x[n2], x[5 + n2], x[10 + n2], x[15 + n2], x[20 + n2]};
-      dft64_prime<5>(t, [&](int k1, double2 v) {
-        u[k1][n2] = k1 * n2 == 0 ? v : cmul64(v, make_double2(kcosd<25>(k1 * n2), -ksind<25>(k1 * n2)));
-      });
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < 5; ++k1) dft64_prime<5>(u[k1], [&](int k2, double2 v) { st(k1 + 5 * k2, v); });
-  } else {
-    dft64_prime<R>(x, st);
   }
 }
 
@@ -190,7 +81,7 @@ __global__ void __launch_bounds__(kPassThreads) pass64_kernel(const double2* __r
         v[s] = make_double2(two & 2u ? hi : lo, two & 1u ? hi : lo);
       }
       double2* o = s_out + threadIdx.x * (R + 1);
-      dft64<R>(v, [&](int r, double2 y) { o[r] = y; });
+      mr_dft<R>(v, [&](int r, double2 y) { o[r] = y; });
     } else {
       const unsigned q = j / Ns, k = j - q * Ns, b = k * (L / (Ns * R));  // twiddle of s: W_L^{s b}
       const double2* x = in + seq + j;
@@ -208,12 +99,12 @@ __global__ void __launch_bounds__(kPassThreads) pass64_kernel(const double2* __r
 #pragma unroll
         for (int s = 0; s < G; ++s) {
           if (g + s >= R || g + s == 0) continue;
-          const double2 w = s == 0 ? h : g == 0 ? lowp[s] : cmul64(h, lowp[s]);
-          v[g + s] = cmul64(v[g + s], w);
+          const double2 w = s == 0 ? h : g == 0 ? lowp[s] : mr_cmul(h, lowp[s]);
+          v[g + s] = mr_cmul(v[g + s], w);
         }
       }
       double2* y = out + seq + (size_t)q * Ns * R + k;
-      dft64<R>(v, [&](int r, double2 t) { y[(size_t)r * Ns] = t; });
+      mr_dft<R>(v, [&](int r, double2 t) { y[(size_t)r * Ns] = t; });
     }
   }
   if constexpr (FIRST) {
@@ -246,52 +137,6 @@ __global__ void __launch_bounds__(256) pass_any_kernel(const double2* __restrict
     }
     out[i] = acc;
   }
-}
-
-// radices of L in pass order: the power of two in as few parts of at most 32
-// as there can be, then the odd primes, 3 with 11 or 5 and 5 with 5 together;
-// false when a prime factor exceeds kMaxRadix
-bool factorise(long long L, std::vector<int>* radices) {
-  radices->clear();
-  long long m = L;
-  int twos = 0;
-  while (m % 2 == 0) {
-    m /= 2;
-    ++twos;
-  }
-  for (int parts = (twos + 4) / 5; parts > 0; --parts) {
-    const int t = (twos + parts - 1) / parts;
-    radices->push_back(1 << t);
-    twos -= t;
-  }
-  std::vector<int> odd;
-  for (long long p = 3; p * p <= m || m > 1; p += 2) {
-    if (p * p > m) p = m;  // m is prime
-    while (m % p == 0) {
-      if (p > kMaxRadix) return false;
-      odd.push_back((int)p);
-      m /= p;
-    }
-    if (m == 1) break;
-  }
-  auto pair = [&](int p, int q) {
-    for (;;) {
-      size_t i = odd.size(), k = odd.size();
-      for (size_t t = 0; t < odd.size(); ++t) {
-        if (odd[t] == p && i == odd.size()) i = t;
-        else if (odd[t] == q) k = t;
-      }
-      if (i == odd.size() || k == odd.size()) return;
-      odd.erase(odd.begin() + (i > k ? i : k));
-      odd.erase(odd.begin() + (i > k ? k : i));
-      radices->push_back(p * q);
-    }
-  };
-  pair(5, 5);
-  pair(3, 11);
-  pair(3, 5);
-  for (int p : odd) radices->push_back(p);
-  return true;
 }
 
 int grid_for(long long work, int num_sms) {
@@ -378,12 +223,12 @@ __global__ void chirp_filter64_kernel(const double2* __restrict__ c, long long L
 __global__ void premul64_kernel(const double2* __restrict__ x, const double2* __restrict__ c, long long L, long long M,
                                 double2* __restrict__ y) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (long long)gridDim.x * blockDim.x)
-    y[i] = i < L ? cmul64(x[i], c[i]) : make_double2(0.0, 0.0);
+    y[i] = i < L ? mr_cmul(x[i], c[i]) : make_double2(0.0, 0.0);
 }
 // conj(a * b): the inverse transform of the product runs as a forward one
 __global__ void conjmul64_kernel(double2* __restrict__ a, const double2* __restrict__ b, long long M) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (long long)gridDim.x * blockDim.x) {
-    const double2 v = cmul64(a[i], b[i]);
+    const double2 v = mr_cmul(a[i], b[i]);
     a[i] = make_double2(v.x, -v.y);
   }
 }
@@ -392,7 +237,7 @@ __global__ void postmul64_kernel(const double2* __restrict__ y, const double2* _
   const double inv = 1.0 / (double)M;
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < L; k += (long long)gridDim.x * blockDim.x) {
     const double2 v = make_double2(y[k].x * inv, -y[k].y * inv);  // conj of the forward transform, / M
-    out[k] = cmul64(v, c[k]);
+    out[k] = mr_cmul(v, c[k]);
   }
 }
 
@@ -435,13 +280,13 @@ __global__ void __launch_bounds__(256) real_power_kernel(const double2* __restri
     double2 w;  // exp(-i pi k / L)
     if (tw) {
       w = __ldg(tw + k / 2);
-      if (k & 1u) w = cmul64(w, w1);
+      if (k & 1u) w = mr_cmul(w, w1);
     } else {
       double s, c;
       sincospi((double)k / (double)L, &s, &c);
       w = make_double2(c, -s);
     }
-    const double2 wo = cmul64(w, o);
+    const double2 wo = mr_cmul(w, o);
     // X[k] = e - i w o; X[L - k] = conj(e) - i conj(w o)
     const double ar = e.x + wo.y, ai = e.y - wo.x;
     put(k, ar * ar + ai * ai);
@@ -466,7 +311,7 @@ long long next_pow2(long long v) {
 size_t fft64_workspace_bytes(long long n, int batch) {
   const long long L = n / 2;
   std::vector<int> r;
-  if (factorise(L, &r)) return (size_t)L * 16;  // the twiddle table
+  if (mr_radices(L, kMaxRadix, &r)) return (size_t)L * 16;  // the twiddle table
   const long long M = next_pow2(2 * L - 1);
   return (size_t)(M + L + 3 * M) * 16;  // table of M, chirp, filter spectrum, two work buffers
 }
@@ -487,7 +332,7 @@ cudaError_t real_power_spectrum(const uint8_t* d_bits, size_t row_bytes, const d
   std::vector<int> radices;
   double2* Z = nullptr;
   const double2* tw = nullptr;
-  if (factorise(L, &radices)) {
+  if (mr_radices(L, kMaxRadix, &radices)) {
     // L is a multiple of 4, so the first radix is a power of two, at least 4
     twiddle64_kernel<<<grid_for(L, num_sms), 256, 0, st>>>(work, L);
     kernel_launch_add(1);
@@ -497,7 +342,7 @@ cudaError_t real_power_spectrum(const uint8_t* d_bits, size_t row_bytes, const d
   } else {
     // Bluestein per sequence: convolution length M = 2^m >= 2L - 1
     const long long M = next_pow2(2 * L - 1);
-    factorise(M, &radices);
+    mr_radices(M, kMaxRadix, &radices);
     double2* twM = work;
     double2* chirp = twM + M;
     double2* H = chirp + L;

@@ -8,16 +8,25 @@
 // with the conjugated code spectrum, inverse FFT, |.|/sqrt(N), last-max
 // argmax; then the hypothesis / bin reduction and the second peak.
 //
-// FFTs of arbitrary length use Bluestein's chirp-z identity
-//   X[k] = w[k] * sum_n (x[n] w[n]) conj(w[k-n]),  w[n] = exp(i s pi n^2 / N)
-// evaluated as a circular convolution of length M = 2^m >= 2N-1 with a radix-2
-// Stockham FFT (Govindaraju et al., SC'08 formulation).
+// A length whose prime factors are at most kGenPrime (the usual ones: 32000 =
+// 2^8 5^3 at 16 MHz) is transformed as it is, by mixed-radix Stockham passes
+// with one butterfly per thread (mixed_radix.cuh).  Any other length uses
+// Bluestein's chirp-z identity
+//   X[k] = w[k] * sum_n (x[n] w[n]) conj(w[k-n]),  w[n] = exp(-i pi n^2 / N)
+// evaluated as a circular convolution of length M = 2^m >= 2N-1 with the same
+// passes.  Inverse transforms run as forward ones of conjugated data (only
+// the magnitude of their results is used).  What bounds a call is the number
+// of launches and, at tens of MB, L2: one GPS search at 16 MHz took 1.29 ms in
+// 150 launches (every transform by Bluestein over radix-2 passes), and takes
+// 0.12 ms in 13.  RMS error of the peaks against 64 bits 1.8e-7 -> 7e-8.
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "dft.cuh"
 #include "engine.h"
+#include "mixed_radix.cuh"
 
 namespace tga {
 
@@ -25,189 +34,265 @@ namespace tga {
 
 namespace {
 
-struct Ws {  // workspace views (float2 units unless noted)
-  float2 *w, *Hf, *Hi, *tw, *C, *X, *Y, *buf, *tmp;
+constexpr int kGenPrime = 64;  // largest prime factor of a direct transform
+
+// Workspace: two buffers of the transforms' batch (length F = N, or the
+// Bluestein length M), twiddles W_F^m, and for Bluestein the chirp and its
+// filter's spectrum.
+struct Ws {
+  float2 *tw, *a, *b, *w, *H;
 };
 
-Ws carve(float2* base, int N, int M, int nb) {
+bool direct_length(int N) {
+  std::vector<int> r;
+  return mr_radices(N, kGenPrime, &r);
+}
+
+Ws carve(float2* base, const GenericPlan& gp, int nb) {
+  const size_t N = gp.N, F = direct_length(gp.N) ? N : (size_t)gp.Mpow2, batch = 2 * (size_t)nb + 2;
   Ws v;
   float2* p = base;
+  v.tw = p; p += F;
+  v.a = p; p += batch * F;
+  v.b = p; p += batch * F;
   v.w = p; p += N;
-  v.Hf = p; p += M;
-  v.Hi = p; p += M;
-  v.tw = p; p += M / 2;
-  v.C = p; p += 2 * (size_t)N;
-  v.X = p; p += (size_t)nb * N;
-  v.Y = p; p += (size_t)2 * nb * N;
-  const int batch = 2 * nb > 2 ? 2 * nb : 2;
-  v.buf = p; p += (size_t)batch * M;
-  v.tmp = p; p += (size_t)batch * M;
+  v.H = p;
   return v;
 }
 
-__global__ void chirp_kernel(int N, int M, float2* w, float2* tw) {
+// tw[m] = exp(-2 pi i m / F)
+__global__ void twiddle_kernel(int F, float2* __restrict__ tw) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < N) {
-    // exp(-i pi n^2 / N) with n^2 reduced mod 2N exactly in integers
-    const long long r = ((long long)i * i) % (2LL * N);
-    double s, c;
-    sincospi((double)r / (double)N, &s, &c);
-    w[i] = make_float2((float)c, (float)-s);
-  }
-  if (i < M / 2) {
-    double s, c;
-    sincospi(2.0 * (double)i / (double)M, &s, &c);
-    tw[i] = make_float2((float)c, (float)-s);  // exp(-2 pi i j / M)
-  }
+  if (i >= F) return;
+  double s, c;
+  sincospi(2.0 * (double)i / (double)F, &s, &c);
+  tw[i] = make_float2((float)c, (float)-s);
 }
 
-// h[m] = conj(w_sigma[m]) wrapped onto the length-M circle; sigma<0 forward.
-__global__ void chirp_filter_kernel(int N, int M, const float2* w, int inverse, float2* h) {
+__global__ void chirp_kernel(int N, float2* __restrict__ w) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  // exp(-i pi n^2 / N) with n^2 reduced mod 2N exactly in integers
+  const long long r = ((long long)i * i) % (2LL * N);
+  double s, c;
+  sincospi((double)r / (double)N, &s, &c);
+  w[i] = make_float2((float)c, (float)-s);
+}
+
+// h[m] = conj(w[m]) wrapped onto the length-M circle
+__global__ void chirp_filter_kernel(int N, int M, const float2* __restrict__ w, float2* __restrict__ h) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   int n = -1;
   if (m < N) n = m;
   else if (m > M - N) n = M - m;
-  float2 v = make_float2(0.f, 0.f);
-  if (n >= 0) {
-    const float2 ws = inverse ? make_float2(w[n].x, -w[n].y) : w[n];  // w_sigma
-    v = make_float2(ws.x, -ws.y);                                   // conj
+  h[m] = n >= 0 ? make_float2(w[n].x, -w[n].y) : make_float2(0.f, 0.f);
+}
+
+// One Stockham pass of radix R (see fft64.cu), one butterfly per thread;
+// blockIdx.y is the sequence.  A pass with Ns = 1 of a power-of-two radix puts
+// its block's R contiguous outputs per thread in order through shared memory.
+constexpr int kGenThreads = 128;
+
+template <int R, bool STAGE>
+__global__ void __launch_bounds__(kGenThreads) pass32_kernel(const float2* __restrict__ in, float2* __restrict__ out,
+                                                             const float2* __restrict__ tw, unsigned L, unsigned Ns) {
+  extern __shared__ float2 s_out[];
+  const unsigned LR = L / R, j = blockIdx.x * kGenThreads + threadIdx.x;
+  const size_t seq = (size_t)blockIdx.y * L;
+  if (j < LR) {
+    float2 v[R];
+    const float2* x = in + seq + j;
+#pragma unroll
+    for (int s = 0; s < R; ++s) v[s] = x[(size_t)s * LR];
+    if constexpr (STAGE) {
+      float2* o = s_out + threadIdx.x * (R + 1);
+      mr_dft<R>(v, [&](int r, float2 y) { o[r] = y; });
+    } else {
+      const unsigned q = j / Ns, k = j - q * Ns, b = k * (L / (Ns * R));  // twiddle of s: W_L^{s b}
+#pragma unroll
+      for (int s = 1; s < R; ++s) v[s] = mr_cmul(v[s], __ldg(tw + (size_t)s * b));
+      float2* y = out + seq + (size_t)q * Ns * R + k;
+      mr_dft<R>(v, [&](int r, float2 t) { y[(size_t)r * Ns] = t; });
+    }
   }
-  h[m] = v;
+  if constexpr (STAGE) {
+    __syncthreads();
+    const unsigned j0 = blockIdx.x * kGenThreads;
+    if (j0 < LR) {
+      const unsigned n = min((unsigned)kGenThreads, LR - j0) * R;
+      float2* y = out + seq + (size_t)j0 * R;
+      for (unsigned i = threadIdx.x; i < n; i += kGenThreads) y[i] = s_out[i + i / R];
+    }
+  }
 }
 
-__global__ void stockham_r2(const float2* __restrict__ x, float2* __restrict__ y, int M, int Ns, long long total,
-                            const float2* __restrict__ tw, int inverse) {
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= total) return;
-  const int half = M >> 1;
-  const long long s = j / half;
-  const int jj = (int)(j - s * half);
-  const int k = jj & (Ns - 1);
-  float2 t = tw[(long long)k * (M / (2 * Ns))];
-  if (inverse) t.y = -t.y;
-  const float2* xs = x + s * M;
-  float2* ys = y + s * M;
-  const float2 a = xs[jj];
-  const float2 b = cmul(xs[jj + half], t);
-  const int idx = (jj - k) * 2 + k;
-  ys[idx] = cadd(a, b);
-  ys[idx + Ns] = csub(a, b);
+// One pass of any radix R, one output per thread (an R-term sum).
+__global__ void __launch_bounds__(256) pass32_any_kernel(const float2* __restrict__ in, float2* __restrict__ out,
+                                                         const float2* __restrict__ tw, unsigned L, int R,
+                                                         unsigned Ns) {
+  const unsigned o = blockIdx.x * 256 + threadIdx.x;
+  if (o >= L) return;
+  const unsigned LR = L / R, NsR = Ns * R, q = o / NsR, rem = o - q * NsR, r = rem / Ns, k = rem - r * Ns;
+  const float2* x = in + (size_t)blockIdx.y * L + q * Ns + k;
+  const unsigned base = (k + r * Ns) * (L / NsR);  // < L
+  float2 acc = make_float2(0.f, 0.f);
+  unsigned m = 0;
+  for (int s = 0; s < R; ++s) {
+    const float2 u = x[(size_t)s * LR], w = __ldg(tw + m);
+    acc.x += u.x * w.x - u.y * w.y;
+    acc.y += u.x * w.y + u.y * w.x;
+    m += base;
+    if (m >= L) m -= L;
+  }
+  out[(size_t)blockIdx.y * L + o] = acc;
 }
 
-// returns pointer holding the result (x or y)
-float2* fft_pow2(float2* x, float2* y, int M, int log2M, int nseq, const float2* tw, int inverse, cudaStream_t st,
-                 cudaError_t* err) {
-  const long long total = (long long)nseq * (M / 2);
-  const int threads = 256;
-  const unsigned blocks = (unsigned)((total + threads - 1) / threads);
-  for (int p = 0, Ns = 1; p < log2M; ++p, Ns <<= 1) {
-    stockham_r2<<<blocks, threads, 0, st>>>(x, y, M, Ns, total, tw, inverse);
+template <int R, bool STAGE>
+cudaError_t run_pass32(const float2* x, float2* y, const float2* tw, int L, int batch, int Ns, cudaStream_t st) {
+  const dim3 grid((unsigned)((L / R + kGenThreads - 1) / kGenThreads), (unsigned)batch);
+  const size_t smem = STAGE ? (size_t)kGenThreads * (R + 1) * sizeof(float2) : 0;
+  pass32_kernel<R, STAGE><<<grid, kGenThreads, smem, st>>>(x, y, tw, (unsigned)L, (unsigned)Ns);
+  return cudaGetLastError();
+}
+
+// forward transforms of `batch` sequences of length L in x (ping-pong with y);
+// *result is the buffer holding them
+cudaError_t fft32(float2* x, float2* y, const float2* tw, int L, int batch, const std::vector<int>& radices,
+                  cudaStream_t st, float2** result) {
+  int Ns = 1;
+  for (int R : radices) {
+    cudaError_t e;
+    switch (R) {
+#define TGA_PASS(RR)                                               \
+  case RR:                                                         \
+    e = run_pass32<RR, false>(x, y, tw, L, batch, Ns, st);         \
+    break;
+#define TGA_PASS2(RR)                                              \
+  case RR:                                                         \
+    e = Ns == 1 ? run_pass32<RR, true>(x, y, tw, L, batch, Ns, st) \
+                : run_pass32<RR, false>(x, y, tw, L, batch, Ns, st); \
+    break;
+      TGA_PASS2(32) TGA_PASS2(16) TGA_PASS2(8) TGA_PASS2(4) TGA_PASS2(2)
+      TGA_PASS(33) TGA_PASS(25) TGA_PASS(15) TGA_PASS(31) TGA_PASS(13) TGA_PASS(11) TGA_PASS(7) TGA_PASS(5) TGA_PASS(3)
+#undef TGA_PASS
+#undef TGA_PASS2
+      default:
+        pass32_any_kernel<<<dim3((unsigned)((L + 255) / 256), (unsigned)batch), 256, 0, st>>>(x, y, tw, (unsigned)L, R,
+                                                                                             (unsigned)Ns);
+        e = cudaGetLastError();
+    }
     kernel_launch_add(1);
+    if (e != cudaSuccess) return e;
+    Ns *= R;
     float2* t = x;
     x = y;
     y = t;
   }
-  *err = cudaGetLastError();
-  return x;
+  *result = x;
+  return cudaSuccess;
 }
 
-__global__ void premul_kernel(const float2* __restrict__ in, int N, int M, long long total, const float2* __restrict__ w,
-                              int inverse, float2* __restrict__ out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const long long s = i / M;
-  const int m = (int)(i - s * M);
-  float2 v = make_float2(0.f, 0.f);
-  if (m < N) {
-    const float2 ws = inverse ? make_float2(w[m].x, -w[m].y) : w[m];
-    v = cmul(in[s * N + m], ws);
-  }
-  out[i] = v;
+// (x w, padded to M) for Bluestein
+__global__ void premul_kernel(const float2* __restrict__ in, int N, int M, const float2* __restrict__ w,
+                              float2* __restrict__ out) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= M) return;
+  const size_t s = blockIdx.y;
+  out[s * M + m] = m < N ? cmul(in[s * N + m], w[m]) : make_float2(0.f, 0.f);
 }
 
-__global__ void pointwise_kernel(float2* __restrict__ a, const float2* __restrict__ h, int M, long long total) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  a[i] = cmul(a[i], h[i % M]);
+// conj(a h): the inverse transform of the product runs as a forward one
+__global__ void pointwise_kernel(float2* __restrict__ a, const float2* __restrict__ h, int M) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= M) return;
+  float2* p = a + (size_t)blockIdx.y * M + m;
+  const float2 v = cmul(*p, h[m]);
+  *p = make_float2(v.x, -v.y);
 }
 
-__global__ void postmul_kernel(const float2* __restrict__ c, int N, int M, long long total, const float2* __restrict__ w,
-                               int inverse, float2* __restrict__ out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const long long s = i / N;
-  const int k = (int)(i - s * N);
-  const float2 ws = inverse ? make_float2(w[k].x, -w[k].y) : w[k];
-  const float2 v = cmul(c[s * M + k], ws);
+__global__ void postmul_kernel(const float2* __restrict__ c, int N, int M, const float2* __restrict__ w,
+                               float2* __restrict__ out) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= N) return;
+  const size_t s = blockIdx.y;
+  const float2 u = c[s * M + k];
+  const float2 v = cmul(make_float2(u.x, -u.y), w[k]);
   const float inv = 1.0f / (float)M;  // M is a power of two: exact
-  out[i] = make_float2(v.x * inv, v.y * inv);
+  out[s * N + k] = make_float2(v.x * inv, v.y * inv);
 }
 
 unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// Unnormalised DFT of nseq sequences of length N (in -> out), forward or inverse.
-cudaError_t bluestein(const GenericPlan& gp, const Ws& v, const float2* in, float2* out, int nseq, int inverse,
-                      cudaStream_t st) {
+// Forward DFTs of nseq sequences of length N held in v.a (direct: of length N
+// each, transformed in place of it; Bluestein: read from `in`); *result is
+// where they are, N apart.
+struct Transform {
+  bool direct;
+  std::vector<int> radices;  // of N, or of M
+};
+cudaError_t transform(const GenericPlan& gp, const Transform& t, const Ws& v, float2* in, float2* spare, int nseq,
+                      cudaStream_t st, float2** result) {
   const int N = gp.N, M = gp.Mpow2;
-  const long long tot = (long long)nseq * M;
-  premul_kernel<<<nblk(tot, 256), 256, 0, st>>>(in, N, M, tot, v.w, inverse, v.buf);
-  kernel_launch_add(1);
+  if (t.direct) return fft32(in, spare, v.tw, N, nseq, t.radices, st, result);
+  // `in` and `spare` have room for nseq sequences of M
   cudaError_t e;
-  float2* r = fft_pow2(v.buf, v.tmp, M, gp.log2M, nseq, v.tw, 0, st, &e);
-  if (e != cudaSuccess) return e;
-  pointwise_kernel<<<nblk(tot, 256), 256, 0, st>>>(r, inverse ? v.Hi : v.Hf, M, tot);
-  kernel_launch_add(1);
-  float2* other = (r == v.buf) ? v.tmp : v.buf;
-  float2* r2 = fft_pow2(r, other, M, gp.log2M, nseq, v.tw, 1, st, &e);
-  if (e != cudaSuccess) return e;
-  const long long totN = (long long)nseq * N;
-  postmul_kernel<<<nblk(totN, 256), 256, 0, st>>>(r2, N, M, totN, v.w, inverse, out);
-  return TGA_GLAUNCHED();
+  const dim3 gm(nblk(M, 256), (unsigned)nseq), gn(nblk(N, 256), (unsigned)nseq);
+  premul_kernel<<<gm, 256, 0, st>>>(in, N, M, v.w, spare);
+  float2* r = nullptr;
+  if ((e = fft32(spare, in, v.tw, M, nseq, t.radices, st, &r)) != cudaSuccess) return e;
+  pointwise_kernel<<<gm, 256, 0, st>>>(r, v.H, M);
+  float2* q = nullptr;
+  if ((e = fft32(r, r == in ? spare : in, v.tw, M, nseq, t.radices, st, &q)) != cudaSuccess) return e;
+  *result = q == in ? spare : in;
+  postmul_kernel<<<gn, 256, 0, st>>>(q, N, M, v.w, *result);
+  kernel_launch_add(3);
+  return cudaGetLastError();
 }
 
-__global__ void code_in_kernel(const float* __restrict__ a, const float* __restrict__ b, int N, float2* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  out[i] = make_float2(a[i], 0.f);
-  out[N + i] = make_float2(b[i], 0.f);
+// Inputs of the forward transforms: sequences 0 and 1 the codes [c,c] and
+// [c,-c] (sample n the (sub)chip floor(n / spc), the sign changing at `split`;
+// correlate.rs:47-58, acquisition.rs:146-159 in f64 as there), 2 + b the signal
+// wiped off for bin b (correlate.rs:110-115, f32 phase)
+__global__ void inputs_kernel(GenericCode code, const float* __restrict__ sig, const double* __restrict__ pp,
+                              const double* __restrict__ fc, int N, float2* __restrict__ X) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+  if (n >= N) return;
+  float2 v;
+  if (q < 2) {
+    const long long i = (long long)floor((double)n / code.spc) % code.len;
+    int c = __ldg(code.chips + (code.boc ? i >> 1 : i));
+    if (code.boc && (i & 1)) c = -c;
+    v = make_float2(q == 1 && n >= code.split ? (float)-c : (float)c, 0.f);
+  } else {
+    const float ph = __double2float_rn(pp[n] * fc[q - 2]);
+    float sn, cs;
+    sincos_phase(ph, &sn, &cs);
+    const float s = sig[n];
+    v = make_float2(cs * s, sn * s);
+  }
+  X[(size_t)q * N + n] = v;
 }
 
-__global__ void conj_kernel(float2* a, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i].y = -a[i].y;
+// conj(X_b conj(C_h)) for every bin b and hypothesis h (q = 2 b + h): the
+// magnitudes of its forward transform are those of the inverse transform of
+// the product
+__global__ void hyp_product_kernel(const float2* __restrict__ X, int N, float2* __restrict__ Y) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+  if (n >= N) return;
+  const float2 c = X[(size_t)(q & 1) * N + n], x = X[(size_t)(2 + (q >> 1)) * N + n];
+  const float2 v = cmul(x, make_float2(c.x, -c.y));
+  Y[(size_t)q * N + n] = make_float2(v.x, -v.y);
 }
 
-// correlate.rs:110-115 (carrier wipe-off, f32 phase)
-__global__ void wipe_kernel(const float* __restrict__ sig, const double* __restrict__ pp, const double* __restrict__ fc,
-                            int N, int nb, float2* __restrict__ X) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)nb * N) return;
-  const int b = (int)(i / N), n = (int)(i - (long long)b * N);
-  const float ph = __double2float_rn(pp[n] * fc[b]);
-  float sn, cs;
-  sincos_phase(ph, &sn, &cs);
-  const float s = sig[n];
-  X[i] = make_float2(cs * s, sn * s);
-}
-
-__global__ void hyp_product_kernel(const float2* __restrict__ X, const float2* __restrict__ C, int N, int nb,
-                                   float2* __restrict__ Y) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)2 * nb * N) return;
-  const long long q = i / N;  // q = b*2 + h
-  const int n = (int)(i - q * N);
-  const int b = (int)(q >> 1), h = (int)(q & 1);
-  Y[i] = cmul(X[(long long)b * N + n], C[(long long)h * N + n]);
-}
-
-// |.| * 1/sqrt(N) and last-max argmax per (bin, hypothesis) row.
-__global__ void norm_argmax_kernel(const float2* __restrict__ Y, int N, float* __restrict__ corr,
-                                   unsigned long long* __restrict__ keys) {
-  const long long q = blockIdx.x;
+// |.| * 1/sqrt(N) and last-max argmax per (bin, hypothesis) row (keys zeroed).
+__global__ void __launch_bounds__(256) norm_argmax_kernel(const float2* __restrict__ Y, int N,
+                                                          float* __restrict__ corr,
+                                                          unsigned long long* __restrict__ keys) {
+  const size_t q = blockIdx.y;
   const float scale = 1.0f / sqrtf((float)N);
   unsigned long long best = 0ull;
-  for (int n = threadIdx.x; n < N; n += blockDim.x) {
+  for (int n = blockIdx.x * 256 + threadIdx.x; n < N; n += gridDim.x * 256) {
     const float2 v = Y[q * N + n];
     const float c = hypotf(v.x, v.y) * scale;  // Complex::norm() * scale
     corr[q * N + n] = c;
@@ -218,13 +303,12 @@ __global__ void norm_argmax_kernel(const float2* __restrict__ Y, int N, float* _
     const unsigned long long t = __shfl_xor_sync(0xffffffffu, best, o);
     best = t > best ? t : best;
   }
-  __shared__ unsigned long long part[32];
+  __shared__ unsigned long long part[8];
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = best;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) best = part[w] > best ? part[w] : best;
-    best = part[0] > best ? part[0] : best;
-    keys[q] = best;
+    for (int w = 1; w < 8; ++w) best = part[w] > best ? part[w] : best;
+    if (best) atomicMax(keys + q, best);
   }
 }
 
@@ -234,23 +318,27 @@ __global__ void select_second_kernel(const float* __restrict__ corr, const unsig
                                      float* __restrict__ res_f) {
   __shared__ int s_q, s_idx;
   __shared__ float s_peak;
-  if (threadIdx.x == 0) {
-    float pb = 0.f;
-    int qb = 0, ib = 0;
-    for (int b = 0; b < nb; ++b) {
-      const unsigned long long ka = keys[2 * b], kb = keys[2 * b + 1];
-      const float pa = __uint_as_float((unsigned)(ka >> 32)), pB = __uint_as_float((unsigned)(kb >> 32));
-      const bool useB = pB > pa;  // strict: [c,c] wins ties
-      const float pr = useB ? pB : pa;
-      if (b == 0 || pr >= pb) {  // last maximum over bins
-        pb = pr;
-        qb = 2 * b + (useB ? 1 : 0);
-        ib = (int)(unsigned)((useB ? kb : ka) & 0xffffffffu);
-      }
+  if (threadIdx.x < 32) {
+    // a bin's row is [c,-c]'s only when strictly stronger; the last bin of the
+    // largest value wins
+    unsigned long long best = 0ull;  // (value bits, bin)
+    for (int b = threadIdx.x; b < nb; b += 32) {
+      const unsigned pa = (unsigned)(keys[2 * b] >> 32), pB = (unsigned)(keys[2 * b + 1] >> 32);
+      const unsigned long long k = ((unsigned long long)max(pa, pB) << 32) | (unsigned)b;
+      best = k > best ? k : best;
     }
-    s_q = qb;
-    s_idx = ib;
-    s_peak = pb;
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long t = __shfl_xor_sync(0xffffffffu, best, o);
+      best = t > best ? t : best;
+    }
+    if (threadIdx.x == 0) {
+      const int b = (int)(unsigned)best;
+      const unsigned long long ka = keys[2 * b], kb = keys[2 * b + 1];
+      const bool useB = (unsigned)(kb >> 32) > (unsigned)(ka >> 32);
+      s_q = 2 * b + (useB ? 1 : 0);
+      s_idx = (int)(unsigned)((useB ? kb : ka) & 0xffffffffu);
+      s_peak = __uint_as_float((unsigned)(best >> 32));
+    }
   }
   __syncthreads();
   const int main_cp = s_idx % period;
@@ -299,49 +387,51 @@ cudaError_t launch_bits_to_signal(const uint8_t* d_bits, size_t row_bytes, int r
 }
 
 size_t generic_work_elems(const GenericPlan& gp, int nb) {
-  const size_t N = gp.N, M = gp.Mpow2, batch = 2 * nb > 2 ? 2 * nb : 2;
-  return N + 2 * M + M / 2 + 2 * N + nb * N + 2 * nb * N + 2 * batch * M;
+  const size_t N = gp.N, F = direct_length(gp.N) ? N : (size_t)gp.Mpow2, batch = 2 * (size_t)nb + 2;
+  // twiddles, two buffers, chirp, filter, and the rows' keys at the end
+  return F + 2 * batch * F + N + F + 2 * (size_t)nb;
 }
 
 cudaError_t launch_generic(const GenericPlan& gp, const float* d_sig, const double* d_pp, const double* d_fc, int nb,
-                           const float* d_code_a, const float* d_code_b, int period, double fs, float2* d_work,
-                           size_t work_elems, float* d_corr, int* d_res_i, float* d_res_f, cudaStream_t st) {
+                           const GenericCode& code, int period, double fs, float2* d_work, size_t work_elems,
+                           float* d_corr, int* d_res_i, float* d_res_f, cudaStream_t st) {
   if (work_elems < generic_work_elems(gp, nb)) return cudaErrorInvalidValue;
   const int N = gp.N, M = gp.Mpow2;
-  Ws v = carve(d_work, N, M, nb);
-  const int mx = N > M / 2 ? N : M / 2;
-  chirp_kernel<<<nblk(mx, 256), 256, 0, st>>>(N, M, v.w, v.tw);
-  kernel_launch_add(1);
-  chirp_filter_kernel<<<nblk(M, 256), 256, 0, st>>>(N, M, v.w, 0, v.Hf);
-  kernel_launch_add(1);
-  chirp_filter_kernel<<<nblk(M, 256), 256, 0, st>>>(N, M, v.w, 1, v.Hi);
+  const Ws v = carve(d_work, gp, nb);
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(d_work + generic_work_elems(gp, nb) - 2 * (size_t)nb);
   cudaError_t e;
-  float2* r = fft_pow2(v.Hf, v.buf, M, gp.log2M, 1, v.tw, 0, st, &e);
+  Transform t;
+  t.direct = mr_radices(N, kGenPrime, &t.radices);
+  const int F = t.direct ? N : M;
+  twiddle_kernel<<<nblk(F, 256), 256, 0, st>>>(F, v.tw);
+  kernel_launch_add(1);
+  if (!t.direct) {
+    mr_radices(M, kGenPrime, &t.radices);
+    chirp_kernel<<<nblk(N, 256), 256, 0, st>>>(N, v.w);
+    chirp_filter_kernel<<<nblk(M, 256), 256, 0, st>>>(N, M, v.w, v.a);
+    kernel_launch_add(2);
+    float2* h = nullptr;
+    if ((e = fft32(v.a, v.b, v.tw, M, 1, t.radices, st, &h)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(v.H, h, (size_t)M * sizeof(float2), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
+  }
+  if ((e = cudaMemsetAsync(keys, 0, 2 * (size_t)nb * sizeof(unsigned long long), st)) != cudaSuccess) return e;
+  // code spectra (correlate.rs:47-68), and the wipe-off and forward transform of every bin
+  const dim3 g1(nblk(N, 256), (unsigned)(nb + 2)), g2(nblk(N, 256), (unsigned)(2 * nb));
+  inputs_kernel<<<g1, 256, 0, st>>>(code, d_sig, d_pp, d_fc, N, v.a);
+  float2 *X = nullptr, *Y = nullptr;
+  if ((e = transform(gp, t, v, v.a, v.b, nb + 2, st, &X)) != cudaSuccess) return e;
+  if (X != v.a) {  // the products go where the spectra are not
+    hyp_product_kernel<<<g2, 256, 0, st>>>(X, N, v.a);
+    e = transform(gp, t, v, v.a, v.b, 2 * nb, st, &Y);
+  } else {
+    hyp_product_kernel<<<g2, 256, 0, st>>>(X, N, v.b);
+    e = transform(gp, t, v, v.b, v.a, 2 * nb, st, &Y);
+  }
   if (e != cudaSuccess) return e;
-  if (r != v.Hf) cudaMemcpyAsync(v.Hf, r, (size_t)M * sizeof(float2), cudaMemcpyDeviceToDevice, st);
-  r = fft_pow2(v.Hi, v.buf, M, gp.log2M, 1, v.tw, 0, st, &e);
-  if (e != cudaSuccess) return e;
-  if (r != v.Hi) cudaMemcpyAsync(v.Hi, r, (size_t)M * sizeof(float2), cudaMemcpyDeviceToDevice, st);
-  // code spectra (correlate.rs:47-68): conj(FFT(code)), conj(FFT(alt))
-  code_in_kernel<<<nblk(N, 256), 256, 0, st>>>(d_code_a, d_code_b, N, v.X);
-  kernel_launch_add(1);
-  if ((e = bluestein(gp, v, v.X, v.C, 2, 0, st)) != cudaSuccess) return e;
-  conj_kernel<<<nblk(2LL * N, 256), 256, 0, st>>>(v.C, 2LL * N);
-  kernel_launch_add(1);
-  // wipe-off and forward FFT per bin
-  wipe_kernel<<<nblk((long long)nb * N, 256), 256, 0, st>>>(d_sig, d_pp, d_fc, N, nb, v.X);
-  kernel_launch_add(1);
-  if ((e = bluestein(gp, v, v.X, v.X, nb, 0, st)) != cudaSuccess) return e;
-  hyp_product_kernel<<<nblk(2LL * nb * N, 256), 256, 0, st>>>(v.X, v.C, N, nb, v.Y);
-  kernel_launch_add(1);
-  if ((e = bluestein(gp, v, v.Y, v.Y, 2 * nb, 1, st)) != cudaSuccess) return e;
-  // reuse tmp as keys storage (2*nb u64)
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(v.tmp);
-  norm_argmax_kernel<<<2 * nb, 512, 0, st>>>(v.Y, N, d_corr, keys);
-  kernel_launch_add(1);
+  norm_argmax_kernel<<<dim3(nblk(N, 256 * 16), (unsigned)(2 * nb)), 256, 0, st>>>(Y, N, d_corr, keys);
   select_second_kernel<<<1, 1024, 0, st>>>(d_corr, keys, N, nb, period, (int)ceil(fs / 1.023e6), d_res_i, d_res_f);
-  (void)fs;
-  return TGA_GLAUNCHED();
+  kernel_launch_add(4);
+  return cudaGetLastError();
 }
 
 }  // namespace tga

@@ -901,38 +901,29 @@ tga_result generic_one(tga_ctx* ctx, int c, const float* d_sig, const double* d_
   if (n > (size_t)(1 << 26)) throw InvalidArg("signal too long for the generic path");
   cudaStream_t st = ctx->stream;
   const int nb = (int)fc.size();
-  // code replicas [c..] and [c, -c] split at min(period, n) (correlate.rs:47-58)
-  std::vector<int8_t> code = resampled_code(c, prn, (double)period, n);
-  std::vector<float> ca(n), cb(n);
-  const size_t split = std::min(period, n);
-  for (size_t i = 0; i < n; ++i) {
-    ca[i] = (float)code[i];
-    cb[i] = i < split ? ca[i] : -ca[i];
-  }
-  float* d_ca = (float*)ctx->buf("gen.ca", n * sizeof(float));
-  float* d_cb = (float*)ctx->buf("gen.cb", n * sizeof(float));
-  CK(cudaMemcpyAsync(d_ca, ca.data(), n * sizeof(float), cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(d_cb, cb.data(), n * sizeof(float), cudaMemcpyHostToDevice, st));
-  ctx->h2d += 2 * n * sizeof(float);
+  // the (sub)chips; the kernel makes the replicas [c..] and [c, -c], split at
+  // min(period, n) (correlate.rs:47-58)
+  const std::vector<int8_t>& chips = cached_chips(ctx, c, prn);
+  int8_t* d_chips = (int8_t*)ctx->buf("gen.chips", chips.size());
+  CK(cudaMemcpyAsync(d_chips, chips.data(), chips.size(), cudaMemcpyHostToDevice, st));
+  ctx->h2d += chips.size();
+  GenericCode code;
+  code.chips = d_chips;
+  code.boc = info(c).boc;
+  code.len = (int)chips.size() * (code.boc ? 2 : 1);
+  code.spc = (double)period / (double)code.len;
+  code.split = (int)std::min(period, n);
   GenericPlan gp;
   gp.N = (int)n;
-  gp.Mpow2 = 1;
-  gp.log2M = 0;
-  while (gp.Mpow2 < 2 * gp.N - 1) {
-    gp.Mpow2 <<= 1;
-    gp.log2M++;
-  }
-  if (gp.Mpow2 < 2) {
-    gp.Mpow2 = 2;
-    gp.log2M = 1;
-  }
+  gp.Mpow2 = 2;
+  while (gp.Mpow2 < 2 * gp.N - 1) gp.Mpow2 <<= 1;
   const size_t welems = generic_work_elems(gp, nb);
   float2* d_work = (float2*)ctx->buf("gen.work", welems * sizeof(float2));
   float* d_corr = (float*)ctx->buf("gen.corr", (size_t)2 * nb * n * sizeof(float));
   int* d_ri = (int*)ctx->buf("gen.ri", 4 * sizeof(int));
   float* d_rf = (float*)ctx->buf("gen.rf", 4 * sizeof(float));
   timed(ctx, "generic", 0.0, [&] {
-    return launch_generic(gp, d_sig, d_pp, d_fc, nb, d_ca, d_cb, (int)period, fs, d_work, welems, d_corr, d_ri,
+    return launch_generic(gp, d_sig, d_pp, d_fc, nb, code, (int)period, fs, d_work, welems, d_corr, d_ri,
                           d_rf, st);
   });
   int ri[4];

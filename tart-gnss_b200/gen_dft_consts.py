@@ -3,8 +3,8 @@
 lengths R in {3, 5, 11, 31}, evaluated in double precision and rounded once
 to binary32; each table also as (v, v) float2 pairs, the operand form of the
 packed FP32 instructions (__ffma2_rn) that apply one constant to the real and
-imaginary parts of a complex value at once.  And csrc/dft64_consts.cuh: the
-same functions in double precision for the radices of the f64 FFT."""
+imaginary parts of a complex value at once.  And csrc/mixed_radix_consts.cuh:
+the same functions in both precisions for the radices of the mixed-radix FFTs."""
 import math
 import os
 
@@ -32,13 +32,14 @@ def main():
         out.append("__constant__ float2 kSin%dx2[%d] = {%s};" % (R, R, ", ".join("{%s, %s}" % (fmt(v), fmt(v)) for v in s)))
     open(os.path.join(HERE, "csrc", "dft_consts.cuh"), "w").write("\n".join(out) + "\n")
     out = ["// Generated constants: cos/sin(2*pi*m/R) in double precision (Python math,",
-           "// tart-gnss_b200/gen_dft_consts.py) for the radices of the f64 FFT.", "#pragma once", ""]
+           "// tart-gnss_b200/gen_dft_consts.py) and rounded once to float, for the radices of the", "// mixed-radix FFTs.",
+           "#pragma once", ""]
     for R in (3, 5, 7, 11, 13, 25, 31, 32):
-        out.append("__constant__ double kCosD%d[%d] = {%s};"
-                   % (R, R, ", ".join(repr(math.cos(2 * math.pi * m / R)) for m in range(R))))
-        out.append("__constant__ double kSinD%d[%d] = {%s};"
-                   % (R, R, ", ".join(repr(math.sin(2 * math.pi * m / R)) for m in range(R))))
-    open(os.path.join(HERE, "csrc", "dft64_consts.cuh"), "w").write("\n".join(out) + "\n")
+        for name, f in (("Cos", math.cos), ("Sin", math.sin)):
+            v = [f(2 * math.pi * m / R) for m in range(R)]
+            out.append("__constant__ double k%sD%d[%d] = {%s};" % (name, R, R, ", ".join(repr(x) for x in v)))
+            out.append("__constant__ float k%sF%d[%d] = {%s};" % (name, R, R, ", ".join(fmt(x) for x in v)))
+    open(os.path.join(HERE, "csrc", "mixed_radix_consts.cuh"), "w").write("\n".join(out) + "\n")
 
 
 if __name__ == "__main__":
