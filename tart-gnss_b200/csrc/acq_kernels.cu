@@ -26,6 +26,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <vector>
 
 #include <atomic>
@@ -57,19 +58,25 @@ void kernel_launch_add(int n) { g_launches += n; }
 // ---------------------------------------------------------------------------
 // antenna means: mean of the +-1 samples over the whole row (acquisition.rs:285)
 // ---------------------------------------------------------------------------
-__global__ void antenna_means_kernel(const uint8_t* __restrict__ bits, size_t row_bytes,
-                                     double* __restrict__ mean) {
+// One CTA per row, bound by the latency of its loads: 16-byte words from the
+// first aligned byte on, four of them in flight per thread, and the bytes
+// before and after one by one (a row may start anywhere).  Byte loads for
+// rows off an 8-byte boundary took 141 us in a search where this takes 10.
+__global__ void __launch_bounds__(1024) antenna_means_kernel(const uint8_t* __restrict__ bits, size_t row_bytes,
+                                                             double* __restrict__ mean) {
   const uint8_t* row = bits + (size_t)blockIdx.x * row_bytes;
   unsigned long long ones = 0;
-  const size_t n_words = row_bytes / 8;
-  const bool aligned = (((uintptr_t)row) & 7) == 0;
-  if (aligned) {
-    const unsigned long long* w = reinterpret_cast<const unsigned long long*>(row);
-    for (size_t i = threadIdx.x; i < n_words; i += blockDim.x) ones += __popcll(__ldg(w + i));
-    for (size_t i = n_words * 8 + threadIdx.x; i < row_bytes; i += blockDim.x) ones += __popc(row[i]);
-  } else {
-    for (size_t i = threadIdx.x; i < row_bytes; i += blockDim.x) ones += __popc(row[i]);
+  const size_t head = min(row_bytes, (size_t)(-(uintptr_t)row & 15));
+  const size_t n_words = (row_bytes - head) / 16;
+  const uint4* w = reinterpret_cast<const uint4*>(row + head);
+#pragma unroll 4
+  for (size_t i = threadIdx.x; i < n_words; i += blockDim.x) {
+    const uint4 v = __ldg(w + i);
+    ones += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
   }
+  if (threadIdx.x < head) ones += __popc(row[threadIdx.x]);
+  const size_t tail = head + n_words * 16 + threadIdx.x;
+  if (tail < row_bytes) ones += __popc(row[tail]);
   for (int o = 16; o > 0; o >>= 1) ones += __shfl_xor_sync(0xffffffffu, ones, o);
   __shared__ unsigned long long part[32];
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ones;
@@ -86,7 +93,7 @@ __global__ void antenna_means_kernel(const uint8_t* __restrict__ bits, size_t ro
 cudaError_t launch_antenna_means(const uint8_t* d_bits, int n_rows, size_t row_bytes, double* d_mean,
                                  cudaStream_t st) {
   if (n_rows <= 0) return cudaSuccess;
-  antenna_means_kernel<<<n_rows, 256, 0, st>>>(d_bits, row_bytes, d_mean);
+  antenna_means_kernel<<<n_rows, 1024, 0, st>>>(d_bits, row_bytes, d_mean);
   return TGA_LAUNCHED();
 }
 
@@ -274,20 +281,32 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
   extern __shared__ float2 buf[];
   __shared__ unsigned long long s_key;
   __shared__ unsigned int s_p2;
+  __shared__ bool s_last;
   // CAND with p2rows: for every residue of the row and every warp that
   // scanned it, its four largest |y|^2 as (value bits << 32) | lag, after
   // the transform buffer (TOP_WPS warps per residue)
   constexpr bool TOP = MODE == CAND;
   constexpr int TOP_WPS = NT / 32 / BC >= 1 ? NT / 32 / BC : 1;
+  static_assert(TOP_WPS <= kTopWarps, "lists of a split row");
   unsigned long long* s_res = reinterpret_cast<unsigned long long*>(buf + BC * LC);
   const bool keep_top = TOP && p.p2rows != nullptr;
   const int tid = threadIdx.x;
   const int S = p.S;
   const int groups = INV ? (S + BC - 1) / BC : 1;
-  int n_work = INV ? p.n_items : (p.n_seq + BC - 1) / BC;
-  if (MODE == CAND) n_work = min(n_work, *p.cand_count);
+  // Work units: row w / split, residue groups [g0, g1) of part w % split.  With
+  // fewer rows than CTAs in flight a row's groups are shared out (one row took
+  // its 16 groups of Lc = 10230 one after the other on one SM: 115 us for the
+  // second peak of one PRN, 15 us so, and 133 against 79 us for its 42 rows);
+  // the parts meet in an atomic maximum, which keeps the tie rule (keys order
+  // by value, then lag).  CORR's split comes from the host, which zeroes the
+  // keys; CAND's from the number of rows listed.
+  const int rows = MODE == CAND ? min(p.n_items, *p.cand_count) : p.n_items;
+  const int split = MODE == CAND ? (rows > 0 ? max(1, min(groups, (int)gridDim.x / rows)) : 1) : max(1, p.split);
+  const int n_work = INV ? rows * split : (p.n_seq + BC - 1) / BC;
 
-  for (int w = blockIdx.x; w < n_work; w += gridDim.x) {
+  for (int unit = blockIdx.x; unit < n_work; unit += gridDim.x) {
+    const int w = INV ? unit / split : unit, part = INV ? unit - w * split : 0;
+    const int g0 = INV ? part * groups / split : 0, g1 = INV ? (part + 1) * groups / split : groups;
     int ab_h = 0, prn = 0, tau_star = 0;
     if (MODE == CORR) {
       ab_h = w / p.n_prn;
@@ -322,7 +341,7 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
       s_p2 = 0u;
     }
 
-    for (int g = 0; g < groups; ++g) {
+    for (int g = g0; g < g1; ++g) {
       // sequence of slot s in this group, or -1 when idle
       auto seq_of = [&](int s) -> int {
         if (INV) {
@@ -521,33 +540,57 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
       }
       if ((tid & 31) == 0) atomicMax(&s_key, kbest);
       __syncthreads();
-      if (tid == 0) p.keys[key_at] = s_key;
-      // CAND with p2rows: the row's second peak against its own maximum,
-      // the largest |y|^2 more than chip_width lags (circularly) from it.
-      // At most ceil((2 chip_width + 1) / S) <= 3 lags of a residue lie that
-      // close, so the four largest of each residue (among the lists of the
-      // warps that scanned it) hold it.
-      if (TOP && keep_top && tid < 32) {
-        const unsigned long long kb = s_key;
-        const int tau_star = (int)(unsigned)kb;
-        float p2 = 0.f;
-        if (kb != 0ull)
-          for (int e = tid; e < S * TOP_WPS * 4; e += 32) {
-            const unsigned long long k = s_res[e];
-            int d = (int)(unsigned)k - tau_star;
-            d = d < 0 ? -d : d;
-            if (k != 0ull && min(d, p.P - d) > p.chip_width) p2 = fmaxf(p2, __uint_as_float((unsigned)(k >> 32)));
+      if (tid == 0) {
+        if (split > 1)
+          atomicMax(p.keys + key_at, s_key);
+        else
+          p.keys[key_at] = s_key;
+      }
+      // CAND with p2rows: the row's second peak against its own maximum, the
+      // largest |y|^2 more than chip_width lags (circularly) from it.  At most
+      // ceil((2 chip_width + 1) / S) <= 3 lags of a residue lie that close, so
+      // the four largest of each residue (among the lists of the warps that
+      // scanned it) hold it.  A split row's lists go through global memory, and
+      // the part that finishes last looks at all of them.
+      if (TOP && keep_top) {
+        const int n_top = S * TOP_WPS * 4;
+        unsigned long long* lists = p.top_lists + (size_t)w * n_top;
+        bool mine = true;
+        if (split > 1) {
+          const int e0 = min(g0 * BC, S) * TOP_WPS * 4, e1 = min(g1 * BC, S) * TOP_WPS * 4;
+          for (int e = e0 + tid; e < e1; e += NT) lists[e] = s_res[e];
+          __threadfence();
+          __syncthreads();
+          if (tid == 0) {
+            s_last = atomicAdd(p.top_done + w, 1) == split - 1;
+            __threadfence();
           }
+          __syncthreads();
+          mine = s_last;
+        }
+        if (mine && tid < 32) {
+          const unsigned long long kb = split > 1 ? __ldcg(p.keys + key_at) : s_key;
+          const int tau_star = (int)(unsigned)kb;
+          float p2 = 0.f;
+          if (kb != 0ull)
+            for (int e = tid; e < n_top; e += 32) {
+              const unsigned long long k = split > 1 ? __ldcg(lists + e) : s_res[e];
+              int d = (int)(unsigned)k - tau_star;
+              d = d < 0 ? -d : d;
+              if (k != 0ull && min(d, p.P - d) > p.chip_width) p2 = fmaxf(p2, __uint_as_float((unsigned)(k >> 32)));
+            }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) p2 = fmaxf(p2, __shfl_xor_sync(0xffffffffu, p2, o));
-        if (tid == 0) p.p2rows[key_at] = p2;
+          for (int o = 16; o > 0; o >>= 1) p2 = fmaxf(p2, __shfl_xor_sync(0xffffffffu, p2, o));
+          if (tid == 0) p.p2rows[key_at] = p2;
+        }
       }
     } else if (MODE == SECOND) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) pbest = fmaxf(pbest, __shfl_xor_sync(0xffffffffu, pbest, o));
       if ((tid & 31) == 0) atomicMax(&s_p2, __float_as_uint(pbest));
       __syncthreads();
-      if (tid == 0) p.best[w].p2 = __uint_as_float(s_p2);
+      // (the bin reduction left 0 there)
+      if (tid == 0) atomicMax(reinterpret_cast<int*>(&p.best[w].p2), (int)s_p2);
     }
     __syncthreads();
   }
@@ -605,9 +648,22 @@ static cudaError_t run_pfa(const PfaParams& p, int n_work_slots, int num_sms, cu
   // FWD modes: n_work_slots counts sequences, grouped BC per work unit
   const int n_work = (MODE == FWD_Z || MODE == FWD_D) ? (n_work_slots + C::BC - 1) / C::BC : n_work_slots;
   int grid = num_sms * per_sm;
-  if (grid > n_work) grid = n_work;
+  PfaParams q = p;
+  if (MODE == CORR || MODE == SECOND) {
+    const int groups = (p.S + C::BC - 1) / C::BC;
+    q.split = n_work > 0 ? std::max(1, std::min(groups, grid / n_work)) : 1;
+    if (MODE == CORR && q.split > 1) {
+      e = cudaMemsetAsync(p.keys, 0, (size_t)n_work * sizeof(unsigned long long), st);
+      if (e != cudaSuccess) return e;
+    }
+    if (grid > n_work * q.split) grid = n_work * q.split;
+  } else if (MODE == CAND) {
+    if (grid > kMaxSplitRows) grid = kMaxSplitRows;
+  } else if (grid > n_work) {
+    grid = n_work;
+  }
   if (grid < 1) return cudaSuccess;
-  kern<<<grid, C::NT, smem, st>>>(p);
+  kern<<<grid, C::NT, smem, st>>>(q);
   return TGA_LAUNCHED();
 }
 
@@ -736,11 +792,22 @@ cudaError_t launch_second_peak(const PolyClass& pc, const SearchDims& dims, cons
   return dispatch_pfa<SECOND>(pc, p, p.n_items, num_sms, st);
 }
 
+size_t split_scratch_bytes(const PolyClass& pc) {
+  // per row a counter and S x kTopWarps x 4 list entries
+  return (size_t)kMaxSplitRows * (sizeof(int) + (size_t)pc.S * kTopWarps * 4 * sizeof(unsigned long long));
+}
+
 cudaError_t launch_correlate_listed(const PolyClass& pc, const SearchDims& dims, const float2* d_Z,
                                     const float2* d_D, const int2* d_cand, const int* d_count, int capacity,
-                                    unsigned long long* d_keys, int num_sms, cudaStream_t st, float* d_p2rows,
-                                    int chip_width) {
+                                    unsigned long long* d_keys, int num_sms, cudaStream_t st, void* d_scratch,
+                                    float* d_p2rows, int chip_width) {
   PfaParams p = {};
+  if (d_p2rows) {
+    p.top_lists = static_cast<unsigned long long*>(d_scratch);
+    p.top_done = reinterpret_cast<int*>(p.top_lists + (size_t)kMaxSplitRows * pc.S * kTopWarps * 4);
+    const cudaError_t e = cudaMemsetAsync(p.top_done, 0, kMaxSplitRows * sizeof(int), st);
+    if (e != cudaSuccess) return e;
+  }
   p.p2rows = d_p2rows;
   p.chip_width = chip_width;
   p.z = const_cast<float2*>(d_Z);
@@ -784,71 +851,105 @@ cudaError_t launch_second_from_rows(const SearchDims& dims, int n_hyp, const flo
 // rows alone give the FP32 search's choice under the same tie rules.
 // Rows are [ant][bin][hyp] with n_hyp hypotheses (2 in the drop-in search,
 // 1 in the non-coherent one); a listed row is (its row index, prn).
-__global__ void tc_candidates_kernel(int n_ant, int n_rows, int n_prn, const unsigned long long* __restrict__ keys,
-                                     float keep, int2* __restrict__ cand, int* __restrict__ count) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_ant * n_prn) return;
-  const int ant = i / n_prn, prn = i - ant * n_prn;
+//
+// Both kernels below read one 8-byte key per row and cell, a chain of nb
+// loads in a chain when one thread walks a cell's rows (10 to 30 us; 7 to 10
+// so).  A CTA takes 32 cells, whose keys are neighbours, and kRowLanes warps
+// share their rows.
+constexpr int kRowLanes = 16;
+
+__global__ void __launch_bounds__(32 * kRowLanes)
+    tc_candidates_kernel(int n_ant, int n_rows, int n_prn, const unsigned long long* __restrict__ keys, float keep,
+                         int2* __restrict__ cand, int* __restrict__ count) {
+  __shared__ float s_max[kRowLanes][32];
+  const int i = blockIdx.x * 32 + threadIdx.x;
+  const bool on = i < n_ant * n_prn;
+  const int ant = on ? i / n_prn : 0, prn = on ? i - ant * n_prn : 0;
   const size_t row0 = (size_t)ant * n_rows;
+  auto key = [&](int r) { return __uint_as_float((unsigned)(__ldg(keys + (row0 + r) * n_prn + prn) >> 32)); };
   float kmax = 0.f;
-  for (int r = 0; r < n_rows; ++r)
-    kmax = fmaxf(kmax, __uint_as_float((unsigned)(keys[(row0 + r) * n_prn + prn] >> 32)));
+  if (on) {
+#pragma unroll 4
+    for (int r = threadIdx.y; r < n_rows; r += kRowLanes) kmax = fmaxf(kmax, key(r));
+  }
+  s_max[threadIdx.y][threadIdx.x] = kmax;
+  __syncthreads();
+#pragma unroll
+  for (int y = 0; y < kRowLanes; ++y) kmax = fmaxf(kmax, s_max[y][threadIdx.x]);
   const float t = kmax * keep;
-  for (int r = 0; r < n_rows; ++r)
-    if (__uint_as_float((unsigned)(keys[(row0 + r) * n_prn + prn] >> 32)) >= t)
-      cand[atomicAdd(count, 1)] = make_int2((int)(row0 + r), prn);
+  if (on) {
+#pragma unroll 4
+    for (int r = threadIdx.y; r < n_rows; r += kRowLanes)
+      if (key(r) >= t) cand[atomicAdd(count, 1)] = make_int2((int)(row0 + r), prn);
+  }
 }
 
 cudaError_t launch_tc_candidates(const SearchDims& dims, int n_hyp, const unsigned long long* d_keys, float keep,
                                  int2* d_cand, int* d_count, cudaStream_t st) {
   const int n = dims.n_ant * dims.n_prn;
   if (n <= 0) return cudaSuccess;
-  tc_candidates_kernel<<<(n + 127) / 128, 128, 0, st>>>(dims.n_ant, dims.nb * n_hyp, dims.n_prn, d_keys, keep,
-                                                        d_cand, d_count);
+  tc_candidates_kernel<<<(n + 31) / 32, dim3(32, kRowLanes), 0, st>>>(dims.n_ant, dims.nb * n_hyp, dims.n_prn,
+                                                                      d_keys, keep, d_cand, d_count);
   return TGA_LAUNCHED();
 }
 
 // ---------------------------------------------------------------------------
 // reduction over hypotheses and Doppler bins (correlate.rs:125-154)
 // ---------------------------------------------------------------------------
-__global__ void reduce_bins_kernel(int n_ant, int nb, int n_prn, const unsigned long long* __restrict__ keys,
-                                   BestRow* __restrict__ best) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_ant * n_prn) return;
-  const int ant = i / n_prn, prn = i - ant * n_prn;
-  float pb = -1.f;
-  unsigned long long kb = 0ull;
-  int hb = 0, bb = 0;
-  for (int bin = 0; bin < nb; ++bin) {
-    const size_t ab = (size_t)ant * nb + bin;
-    const unsigned long long ka = keys[(ab * 2 + 0) * n_prn + prn];
-    const unsigned long long kB = keys[(ab * 2 + 1) * n_prn + prn];
-    const float pa = __uint_as_float((unsigned)(ka >> 32)), pB = __uint_as_float((unsigned)(kB >> 32));
-    // hypotheses: [c,-c] replaces [c,c] only when strictly stronger
-    const bool useB = pB > pa;
-    const float pr = useB ? pB : pa;
-    // bins: Iterator::max_by keeps the last maximum
-    if (bin == 0 || pr >= pb) {
-      pb = pr;
-      kb = useB ? kB : ka;
-      hb = useB ? 1 : 0;
-      bb = bin;
+template <int HYP>
+__global__ void __launch_bounds__(32 * kRowLanes)
+    reduce_bins_kernel(int n_ant, int nb, int n_prn, const unsigned long long* __restrict__ keys,
+                       BestRow* __restrict__ best) {
+  __shared__ unsigned long long s_best[kRowLanes][32];
+  const int i = blockIdx.x * 32 + threadIdx.x;
+  const bool on = i < n_ant * n_prn;
+  const int ant = on ? i / n_prn : 0, prn = on ? i - ant * n_prn : 0;
+  auto key = [&](int bin, int h) { return __ldg(keys + (((size_t)ant * nb + bin) * HYP + h) * n_prn + prn); };
+  // (value, bin, hypothesis): the largest is the last bin of the largest
+  // value (Iterator::max_by keeps the last maximum).  A NaN is never above
+  // another value, and nothing is above a NaN in bin 0.
+  unsigned long long top = 0ull;
+  if (on) {
+#pragma unroll 4
+    for (int bin = threadIdx.y; bin < nb; bin += kRowLanes) {
+      float pr = __uint_as_float((unsigned)(key(bin, 0) >> 32));
+      int h = 0;
+      if (HYP == 2) {
+        const float pB = __uint_as_float((unsigned)(key(bin, HYP - 1) >> 32));
+        // hypotheses: [c,-c] replaces [c,c] only when strictly stronger
+        if (pB > pr) pr = pB, h = 1;
+      }
+      const unsigned v = pr >= 0.f ? __float_as_uint(pr) : bin == 0 ? 0xffffffffu : 0u;
+      const unsigned long long k = ((unsigned long long)v << 32) | (unsigned)(bin * 2 + h);
+      if (v != 0u || pr >= 0.f) top = k > top ? k : top;
     }
   }
+  s_best[threadIdx.y][threadIdx.x] = top;
+  __syncthreads();
+  if (threadIdx.y != 0 || !on) return;
+#pragma unroll
+  for (int y = 0; y < kRowLanes; ++y) top = s_best[y][threadIdx.x] > top ? s_best[y][threadIdx.x] : top;
+  const int bin = (int)(unsigned)top >> 1, h = (int)top & 1;
+  const unsigned long long k = key(bin, h);
   BestRow r;
-  r.ab = ant * nb + bb;
-  r.hyp = hb;
-  r.tau = (int)(unsigned)(kb & 0xffffffffull);
-  r.p = pb;
+  r.ab = ant * nb + bin;
+  r.hyp = h;
+  r.tau = (int)(unsigned)(k & 0xffffffffull);
+  r.p = __uint_as_float((unsigned)(k >> 32));
   r.p2 = 0.f;
   best[i] = r;
 }
 
-cudaError_t launch_reduce_bins(const SearchDims& dims, const unsigned long long* d_keys, BestRow* d_best,
+cudaError_t launch_reduce_bins(const SearchDims& dims, int n_hyp, const unsigned long long* d_keys, BestRow* d_best,
                                cudaStream_t st) {
   const int n = dims.n_ant * dims.n_prn;
   if (n <= 0) return cudaSuccess;
-  reduce_bins_kernel<<<(n + 127) / 128, 128, 0, st>>>(dims.n_ant, dims.nb, dims.n_prn, d_keys, d_best);
+  const int grid = (n + 31) / 32;
+  const dim3 block(32, kRowLanes);
+  if (n_hyp == 2)
+    reduce_bins_kernel<2><<<grid, block, 0, st>>>(dims.n_ant, dims.nb, dims.n_prn, d_keys, d_best);
+  else
+    reduce_bins_kernel<1><<<grid, block, 0, st>>>(dims.n_ant, dims.nb, dims.n_prn, d_keys, d_best);
   return TGA_LAUNCHED();
 }
 

@@ -115,8 +115,13 @@ cudaError_t launch_correlate(const PolyClass& pc, const SearchDims& dims, const 
 // launch_second_peak computes for a chosen row) is written there as well.
 cudaError_t launch_correlate_listed(const PolyClass& pc, const SearchDims& dims, const float2* d_Z,
                                     const float2* d_D, const int2* d_cand, const int* d_count, int capacity,
-                                    unsigned long long* d_keys, int num_sms, cudaStream_t st,
+                                    unsigned long long* d_keys, int num_sms, cudaStream_t st, void* d_scratch,
                                     float* d_p2rows = nullptr, int chip_width = 0);
+// Scratch of launch_correlate_listed: it shares a row's residues between CTAs
+// when fewer rows are listed than CTAs run (at most kMaxSplitRows CTAs).
+constexpr int kMaxSplitRows = 512;
+constexpr int kTopWarps = 11;  // most warps that scan one residue for its largest values
+size_t split_scratch_bytes(const PolyClass& pc);
 // d_best[w].p2 = d_p2rows at the row d_best[w] chose (the keys' layout:
 // [ab][hyp][prn] with n_hyp hypotheses, 2 for the drop-in search, 1 for the
 // non-coherent one).
@@ -150,7 +155,9 @@ cudaError_t launch_correlate_tc(const PolyClass& pc, const SearchDims& dims, con
 cudaError_t launch_correlate_tc_nc(const PolyClass& pc, const SearchDims& dims, int B, const void* d_bmat,
                                    const void* d_z16, const void* d_d16, unsigned long long* d_keys, int* d_err,
                                    int test_flags, int num_sms, cudaStream_t st);
-cudaError_t launch_reduce_bins(const SearchDims& dims, const unsigned long long* d_keys,
+// per (antenna, PRN): the last Doppler bin with the largest key, over n_hyp
+// hypotheses (2 in the drop-in search, 1 in the non-coherent one)
+cudaError_t launch_reduce_bins(const SearchDims& dims, int n_hyp, const unsigned long long* d_keys,
                                BestRow* d_best, cudaStream_t st);
 cudaError_t launch_second_peak(const PolyClass& pc, const SearchDims& dims, const float2* d_Z,
                                const float2* d_D, BestRow* d_best, int chip_width, int num_sms,
@@ -245,8 +252,6 @@ cudaError_t launch_nc_frontend(const SampleSource& src, const SearchDims& dims, 
                                long long start, float2* d_z, cudaStream_t st);
 cudaError_t launch_nc_correlate(const PolyClass& pc, const SearchDims& dims, int B, const float2* d_z,
                                 const float2* d_D, unsigned long long* d_keys, int num_sms, cudaStream_t st);
-cudaError_t launch_nc_reduce(const SearchDims& dims, const unsigned long long* d_keys, BestRow* d_best,
-                             cudaStream_t st);
 // launch_nc_correlate over the (ab, prn) rows listed in d_cand (*d_count of
 // them, at most capacity), as the FP32 re-evaluation of a reduced-precision
 // search's candidates: each listed row's key is written where
@@ -256,7 +261,7 @@ cudaError_t launch_nc_reduce(const SearchDims& dims, const unsigned long long* d
 cudaError_t launch_nc_correlate_listed(const PolyClass& pc, const SearchDims& dims, int B, const float2* d_z,
                                        const float2* d_D, const int2* d_cand, const int* d_count, int capacity,
                                        unsigned long long* d_keys, int num_sms, cudaStream_t st,
-                                       float* d_p2rows = nullptr, int chip_width = 0);
+                                       void* d_scratch, float* d_p2rows = nullptr, int chip_width = 0);
 cudaError_t launch_nc_second(const PolyClass& pc, const SearchDims& dims, int B, const float2* d_z,
                              const float2* d_D, BestRow* d_best, int chip_width, int num_sms, cudaStream_t st);
 

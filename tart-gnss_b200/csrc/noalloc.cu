@@ -297,7 +297,7 @@ extern "C" int tga_acquire_single_static(int constellation, const float* d_signa
   if (e == cudaSuccess) e = launch_frontend(src, dims, pc, d_z, st);
   if (e == cudaSuccess) e = launch_forward_z(pc, (int)nb, d_z, sms, st);
   if (e == cudaSuccess) e = launch_correlate(pc, dims, d_z, d_D, d_keys, sms, st);
-  if (e == cudaSuccess) e = launch_reduce_bins(dims, d_keys, d_best, st);
+  if (e == cudaSuccess) e = launch_reduce_bins(dims, 2, d_keys, d_best, st);
   if (e == cudaSuccess) e = launch_second_peak(pc, dims, d_z, d_D, d_best, chip_width, sms, st);
   if (e == cudaSuccess) e = launch_finalize(pc, dims, d_best, center_freq, d_chips + Lc, 0, d_cell, st);
   if (e != cudaSuccess) return TGA_ERR_CUDA;

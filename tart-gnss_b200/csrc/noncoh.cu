@@ -14,6 +14,8 @@
 // center + (i - (nb - 1) / 2) step; the last maximum over bins wins.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include <cstdint>
 
 #include "dft.cuh"
@@ -193,27 +195,38 @@ struct NcParams {
   BestRow* best;             // NC_SECOND: [n_ant][n_prn]
   const int2* cand;          // NC_CAND: the rows
   const int* cand_count;     // NC_CAND: their number (device)
+  int split;                 // NC_PEAK / NC_SECOND: CTAs that share a row's residue groups
+  unsigned long long* top_lists;  // NC_CAND with p2rows, split rows: their residues' lists
+  int* top_done;             // and the parts finished (zeroed), both for kMaxSplitRows rows
   float* p2rows;             // NC_CAND (optional): each row's second peak
                              // against its own maximum, where its key goes
 };
 
-template <int M, int BC, int NT, int MODE>
-__global__ void __launch_bounds__(NT, 1) nc_correlate_kernel(NcParams p) {
+template <int M, int BC, int NT, int MINB, int MODE>
+__global__ void __launch_bounds__(NT, MINB) nc_correlate_kernel(NcParams p) {
   using G = Geo<M>;
   constexpr int COLS = G::COLS, LC = G::LC, NC = G::NC;
   extern __shared__ float2 buf[];
   float* acc = reinterpret_cast<float*>(buf + BC * LC);
   __shared__ unsigned long long s_key;
   __shared__ unsigned int s_p2;
+  __shared__ bool s_last;
   // NC_CAND with p2rows: for every residue and every warp that scanned it,
   // its four largest summed |y|^2 as (value bits << 32) | lag, after acc
   constexpr int TOP_WPS = NT / 32 / BC >= 1 ? NT / 32 / BC : 1;
+  static_assert(TOP_WPS <= kTopWarps, "lists of a split row");
   const bool keep_top = MODE == NC_CAND && p.p2rows != nullptr;
   unsigned long long* s_res = reinterpret_cast<unsigned long long*>(acc + BC * LC);
   const int tid = threadIdx.x, S = p.S;
   const int groups = (S + BC - 1) / BC;
-  const int n_work = MODE == NC_CAND ? min(p.n_items, *p.cand_count) : p.n_items;
-  for (int w = blockIdx.x; w < n_work; w += gridDim.x) {
+  // a row's residue groups are shared between CTAs as in pfa_kernel (32 rows
+  // of two groups: 97 us for the second peaks of 32 PRNs over ten periods on
+  // 32 CTAs, half on 64)
+  const int rows = MODE == NC_CAND ? min(p.n_items, *p.cand_count) : p.n_items;
+  const int split = MODE == NC_CAND ? (rows > 0 ? max(1, min(groups, (int)gridDim.x / rows)) : 1) : p.split;
+  for (int unit = blockIdx.x; unit < rows * split; unit += gridDim.x) {
+    const int w = unit / split, part = unit - w * split;
+    const int g0 = part * groups / split, g1 = (part + 1) * groups / split;
     constexpr bool ARGMAX = MODE == NC_PEAK || MODE == NC_CAND;
     int ab, prn, tau_star = 0;
     if (MODE == NC_PEAK) {
@@ -235,7 +248,7 @@ __global__ void __launch_bounds__(NT, 1) nc_correlate_kernel(NcParams p) {
     }
     unsigned long long kbest = 0ull;
     float pbest = 0.f;
-    for (int g = 0; g < groups; ++g) {
+    for (int g = g0; g < g1; ++g) {
       auto seq_of = [&](int s) -> int {
         const int rho = g * BC + s;
         return rho < S ? rho : -1;
@@ -363,48 +376,75 @@ __global__ void __launch_bounds__(NT, 1) nc_correlate_kernel(NcParams p) {
       }
       if ((tid & 31) == 0) atomicMax(&s_key, kbest);
       __syncthreads();
-      if (tid == 0) p.keys[(size_t)ab * p.n_prn + prn] = s_key;
+      const size_t key_at = (size_t)ab * p.n_prn + prn;
+      if (tid == 0) {
+        if (split > 1)
+          atomicMax(p.keys + key_at, s_key);
+        else
+          p.keys[key_at] = s_key;
+      }
       // NC_CAND with p2rows: the row's second peak against its own maximum
-      // (at most three lags of a residue lie within chip_width of it)
-      if (keep_top && tid < 32) {
-        const unsigned long long kb = s_key;
-        const int tau = (int)(unsigned)kb;
-        float p2 = 0.f;
-        if (kb != 0ull)
-          for (int e = tid; e < S * TOP_WPS * 4; e += 32) {
-            const unsigned long long k = s_res[e];
-            int d = (int)(unsigned)k - tau;
-            d = d < 0 ? -d : d;
-            if (k != 0ull && min(d, p.P - d) > p.chip_width) p2 = fmaxf(p2, __uint_as_float((unsigned)(k >> 32)));
+      // (at most three lags of a residue lie within chip_width of it); of a
+      // split row's parts the last one to finish sees all lists
+      if (keep_top) {
+        const int n_top = S * TOP_WPS * 4;
+        unsigned long long* lists = p.top_lists + (size_t)w * n_top;
+        bool mine = true;
+        if (split > 1) {
+          const int e0 = min(g0 * BC, S) * TOP_WPS * 4, e1 = min(g1 * BC, S) * TOP_WPS * 4;
+          for (int e = e0 + tid; e < e1; e += NT) lists[e] = s_res[e];
+          __threadfence();
+          __syncthreads();
+          if (tid == 0) {
+            s_last = atomicAdd(p.top_done + w, 1) == split - 1;
+            __threadfence();
           }
+          __syncthreads();
+          mine = s_last;
+        }
+        if (mine && tid < 32) {
+          const unsigned long long kb = split > 1 ? __ldcg(p.keys + key_at) : s_key;
+          const int tau = (int)(unsigned)kb;
+          float p2 = 0.f;
+          if (kb != 0ull)
+            for (int e = tid; e < n_top; e += 32) {
+              const unsigned long long k = split > 1 ? __ldcg(lists + e) : s_res[e];
+              int d = (int)(unsigned)k - tau;
+              d = d < 0 ? -d : d;
+              if (k != 0ull && min(d, p.P - d) > p.chip_width) p2 = fmaxf(p2, __uint_as_float((unsigned)(k >> 32)));
+            }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) p2 = fmaxf(p2, __shfl_xor_sync(0xffffffffu, p2, o));
-        if (tid == 0) p.p2rows[(size_t)ab * p.n_prn + prn] = p2;
+          for (int o = 16; o > 0; o >>= 1) p2 = fmaxf(p2, __shfl_xor_sync(0xffffffffu, p2, o));
+          if (tid == 0) p.p2rows[key_at] = p2;
+        }
       }
     } else {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) pbest = fmaxf(pbest, __shfl_xor_sync(0xffffffffu, pbest, o));
       if ((tid & 31) == 0) atomicMax(&s_p2, __float_as_uint(pbest));
       __syncthreads();
-      if (tid == 0) p.best[w].p2 = __uint_as_float(s_p2);
+      // (the bin reduction left 0 there)
+      if (tid == 0) atomicMax(reinterpret_cast<int*>(&p.best[w].p2), (int)s_p2);
     }
     __syncthreads();
   }
 }
 
+// Two CTAs per SM hide each other's barriers where the buffers allow it
+// (32 PRNs x 21 bins x 10 periods of Lc = 1023: 455 us with one, 367 with two).
 template <int M>
 struct NcCfg;
 template <>
 struct NcCfg<1> {
-  static constexpr int BC = 8, NT = 288;
+  static constexpr int BC = 8, NT = 288, MINB = 2;
 };
 template <>
 struct NcCfg<4> {
-  static constexpr int BC = 2, NT = 288;
+  static constexpr int BC = 2, NT = 288, MINB = 2;
 };
 template <>
 struct NcCfg<10> {
-  static constexpr int BC = 1, NT = 352;
+  static constexpr int BC = 1, NT = 352, MINB = 1;
 };
 
 template <int M, int MODE>
@@ -416,16 +456,27 @@ cudaError_t run_nc(const NcParams& p, int num_sms, cudaStream_t st) {
     constexpr int WPS = C::NT / 32 / C::BC >= 1 ? C::NT / 32 / C::BC : 1;
     smem += (size_t)p.S * WPS * 4 * sizeof(unsigned long long);
   }
-  auto kern = nc_correlate_kernel<M, C::BC, C::NT, MODE>;
+  auto kern = nc_correlate_kernel<M, C::BC, C::NT, C::MINB, MODE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, smem);
   if (per_sm < 1) per_sm = 1;
   int grid = num_sms * per_sm;
-  if (grid > p.n_items) grid = p.n_items;
-  if (grid < 1) return cudaSuccess;
-  kern<<<grid, C::NT, smem, st>>>(p);
+  NcParams q = p;
+  if (p.n_items < 1) return cudaSuccess;
+  if (MODE == NC_CAND) {
+    if (grid > kMaxSplitRows) grid = kMaxSplitRows;
+  } else {
+    const int groups = (p.S + C::BC - 1) / C::BC;
+    q.split = std::max(1, std::min(groups, grid / p.n_items));
+    if (MODE == NC_PEAK && q.split > 1) {
+      e = cudaMemsetAsync(p.keys, 0, (size_t)p.n_items * sizeof(unsigned long long), st);
+      if (e != cudaSuccess) return e;
+    }
+    if (grid > p.n_items * q.split) grid = p.n_items * q.split;
+  }
+  kern<<<grid, C::NT, smem, st>>>(q);
   kernel_launch_add(1);
   return cudaGetLastError();
 }
@@ -438,33 +489,6 @@ cudaError_t dispatch_nc(int M, const NcParams& p, int num_sms, cudaStream_t st) 
     case 10: return run_nc<10, MODE>(p, num_sms, st);
   }
   return cudaErrorInvalidValue;
-}
-
-// per (antenna, PRN): the last bin with the largest accumulated peak
-__global__ void nc_reduce_kernel(int n_ant, int nb, int n_prn, const unsigned long long* __restrict__ keys,
-                                 BestRow* __restrict__ best) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_ant * n_prn) return;
-  const int ant = i / n_prn, prn = i - ant * n_prn;
-  float pb = -1.f;
-  unsigned long long kb = 0ull;
-  int bb = 0;
-  for (int bin = 0; bin < nb; ++bin) {
-    const unsigned long long k = keys[((size_t)ant * nb + bin) * n_prn + prn];
-    const float pr = __uint_as_float((unsigned)(k >> 32));
-    if (bin == 0 || pr >= pb) {
-      pb = pr;
-      kb = k;
-      bb = bin;
-    }
-  }
-  BestRow r;
-  r.ab = ant * nb + bb;
-  r.hyp = 0;
-  r.tau = (int)(unsigned)(kb & 0xffffffffull);
-  r.p = pb;
-  r.p2 = 0.f;
-  best[i] = r;
 }
 
 }  // namespace
@@ -517,15 +541,6 @@ cudaError_t launch_nc_correlate(const PolyClass& pc, const SearchDims& dims, int
   return dispatch_nc<NC_PEAK>(pc.M, p, num_sms, st);
 }
 
-cudaError_t launch_nc_reduce(const SearchDims& dims, const unsigned long long* d_keys, BestRow* d_best,
-                             cudaStream_t st) {
-  const int n = dims.n_ant * dims.n_prn;
-  if (n <= 0) return cudaSuccess;
-  nc_reduce_kernel<<<(n + 127) / 128, 128, 0, st>>>(dims.n_ant, dims.nb, dims.n_prn, d_keys, d_best);
-  kernel_launch_add(1);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_nc_second(const PolyClass& pc, const SearchDims& dims, int B, const float2* d_z,
                              const float2* d_D, BestRow* d_best, int chip_width, int num_sms, cudaStream_t st) {
   NcParams p = {};
@@ -543,9 +558,15 @@ cudaError_t launch_nc_second(const PolyClass& pc, const SearchDims& dims, int B,
 
 cudaError_t launch_nc_correlate_listed(const PolyClass& pc, const SearchDims& dims, int B, const float2* d_z,
                                        const float2* d_D, const int2* d_cand, const int* d_count, int capacity,
-                                       unsigned long long* d_keys, int num_sms, cudaStream_t st, float* d_p2rows,
-                                       int chip_width) {
+                                       unsigned long long* d_keys, int num_sms, cudaStream_t st, void* d_scratch,
+                                       float* d_p2rows, int chip_width) {
   NcParams p = {};
+  if (d_p2rows) {
+    p.top_lists = static_cast<unsigned long long*>(d_scratch);
+    p.top_done = reinterpret_cast<int*>(p.top_lists + (size_t)kMaxSplitRows * pc.S * kTopWarps * 4);
+    const cudaError_t e = cudaMemsetAsync(p.top_done, 0, kMaxSplitRows * sizeof(int), st);
+    if (e != cudaSuccess) return e;
+  }
   p.p2rows = d_p2rows;
   p.chip_width = chip_width;
   p.z = d_z;

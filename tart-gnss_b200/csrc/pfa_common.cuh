@@ -133,6 +133,9 @@ struct PfaParams {
   BestRow* best;              // SECOND in/out
   const int2* cand;           // CAND: the rows to evaluate
   const int* cand_count;      // CAND: their number (device)
+  int split;                  // CORR / SECOND: CTAs that share a row's residue groups
+  unsigned long long* top_lists;  // CAND with p2rows, split rows: their residues' lists
+  int* top_done;              // and the parts finished (zeroed), both for kMaxSplitRows rows
   float* p2rows;              // CAND (optional): each listed row's second peak
                               // against its own maximum, where its key goes
   uint4* z16;                 // FWD_Z (optional): the transformed sequences also as TcUnits, x z16_scale

@@ -489,6 +489,7 @@ struct GroupBufs {
   int* count = nullptr;
   // and each re-evaluated row's second peak against its own maximum
   float* p2rows = nullptr;
+  void* scratch = nullptr;  // split_scratch_bytes
 };
 
 GroupBufs prepare_group(tga_ctx* ctx, const ClassGroup& grp, int n_ant, int nb, const std::string& tag) {
@@ -526,6 +527,7 @@ GroupBufs prepare_group(tga_ctx* ctx, const ClassGroup& grp, int n_ant, int nb, 
     b.d16 = ctx->buf(tag + ".d16", tc_operand_bytes(pc, (long long)n_prn * 2));
     b.keys32 = (unsigned long long*)ctx->buf(tag + ".keys32", (size_t)n_ab * 2 * n_prn * sizeof(unsigned long long));
     b.p2rows = (float*)ctx->buf(tag + ".p2rows", (size_t)n_ab * 2 * n_prn * sizeof(float));
+    b.scratch = ctx->buf(tag + ".split", split_scratch_bytes(pc));
     b.cand = (int2*)ctx->buf(tag + ".cand", (size_t)n_ab * 2 * n_prn * sizeof(int2));
     b.count = (int*)ctx->buf(tag + ".count", sizeof(int));
     // DFT matrices of the class (they depend on Lc only), uploaded once per context
@@ -597,7 +599,7 @@ void enqueue_group(tga_ctx* ctx, const ClassGroup& grp, const GroupBufs& b, cons
     // rows need no second transform
     timed(ctx, ("refine" + cls).c_str(), 0.0, [&] {
       return launch_correlate_listed(pc, dims, b.z, b.D, b.cand, b.count, n_ab * 2 * n_prn, b.keys32, ctx->num_sms,
-                                     st, rows_p2 ? b.p2rows : nullptr, chip_width);
+                                     st, b.scratch, rows_p2 ? b.p2rows : nullptr, chip_width);
     });
   } else {
     timed(ctx, ("forward_z" + cls).c_str(), (double)n_ab * 2 * fft_flops(pc.P),
@@ -606,7 +608,7 @@ void enqueue_group(tga_ctx* ctx, const ClassGroup& grp, const GroupBufs& b, cons
           [&] { return launch_correlate(pc, dims, b.z, b.D, b.keys, ctx->num_sms, st); });
   }
   const unsigned long long* keys32 = ctx->precision == TGA_PRECISION_FP16_TC ? b.keys32 : b.keys;
-  timed(ctx, ("reduce_bins" + cls).c_str(), 0.0, [&] { return launch_reduce_bins(dims, keys32, b.best, st); });
+  timed(ctx, ("reduce_bins" + cls).c_str(), 0.0, [&] { return launch_reduce_bins(dims, 2, keys32, b.best, st); });
   if (rows_p2)
     timed(ctx, ("second_peak" + cls).c_str(), 0.0,
           [&] { return launch_second_from_rows(dims, 2, b.p2rows, b.best, st); });
@@ -2078,6 +2080,7 @@ void nc_run_group(tga_ctx* ctx, const uint8_t* d_bits, size_t row_bytes, const d
   void *d_z16 = nullptr, *d_zmap = nullptr, *d_d16 = nullptr, *d_bmat = nullptr;
   int *d_err = nullptr, *d_count = nullptr;
   unsigned long long* d_keys32 = nullptr;
+  void* d_split = nullptr;
   int2* d_cand = nullptr;
   // tensor-core mode takes the second peaks from the FP32 re-evaluation
   // (the four largest sums per residue; exact while at most three lags of a
@@ -2101,6 +2104,7 @@ void nc_run_group(tga_ctx* ctx, const uint8_t* d_bits, size_t row_bytes, const d
     }
     d_keys32 = (unsigned long long*)ctx->buf(tag + ".keys32", n_rows * sizeof(unsigned long long));
     if (rows_p2) d_p2rows = (float*)ctx->buf(tag + ".p2rows", n_rows * sizeof(float));
+    d_split = ctx->buf(tag + ".split", split_scratch_bytes(pc));
     d_cand = (int2*)ctx->buf(tag + ".cand", n_rows * sizeof(int2));
     d_count = (int*)ctx->buf(tag + ".count", (size_t)n_chunks * sizeof(int));
     timed(ctx, ("nc_tc_pack" + cls).c_str(), 0.0,
@@ -2141,13 +2145,13 @@ void nc_run_group(tga_ctx* ctx, const uint8_t* d_bits, size_t row_bytes, const d
       });
       timed(ctx, ("nc_refine" + cls).c_str(), 0.0, [&] {
         return launch_nc_correlate_listed(pc, cd, B, d_z, d_D, d_cand + r0, d_count + ch, na * nb * n_prn,
-                                          d_keys32 + r0, ctx->num_sms, st, rows_p2 ? d_p2rows + r0 : nullptr, cw);
+                                          d_keys32 + r0, ctx->num_sms, st, d_split, rows_p2 ? d_p2rows + r0 : nullptr, cw);
       });
     } else {
       timed(ctx, ("nc_correlate" + cls).c_str(), (double)na * nb * n_prn * B * row,
             [&] { return launch_nc_correlate(pc, cd, B, d_z, d_D, d_keys + r0, ctx->num_sms, st); });
     }
-    timed(ctx, ("nc_reduce" + cls).c_str(), 0.0, [&] { return launch_nc_reduce(cd, (tc ? d_keys32 : d_keys) + r0, cbest, st); });
+    timed(ctx, ("nc_reduce" + cls).c_str(), 0.0, [&] { return launch_reduce_bins(cd, 1, (tc ? d_keys32 : d_keys) + r0, cbest, st); });
     if (rows_p2)
       timed(ctx, ("nc_second" + cls).c_str(), 0.0,
             [&] { return launch_second_from_rows(cd, 1, d_p2rows + r0, cbest, st); });

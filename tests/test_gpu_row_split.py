@@ -1,0 +1,100 @@
+"""Rows whose residue groups are shared between CTAs (few rows in a call): the
+cells of one PRN, one antenna and few bins, searched alone, must equal the same
+cells out of a call with enough rows that no row is shared; residue counts
+below, at and off the groups of every code length.  Numbers of Doppler bins
+around the width of the bin reduction, and recordings whose rows start at
+every byte alignment (each antenna must give the cells of a recording that
+holds it alone).  All equalities are exact: the same FP32 values are compared,
+and ties have one winner.
+"""
+import numpy as np
+import pytest
+
+import tga
+
+pytestmark = pytest.mark.gpu
+FIELDS = ("best_codephase", "best_freq_idx", "hypothesis", "signal_strength", "second_peak", "frequency")
+NC_FIELDS = ("best_codephase", "best_freq_idx", "power", "second_power", "frequency")
+SHAPES = [(tga.GPS, 1023, 1), (tga.GPS, 1023, 8), (tga.GPS, 1023, 9), (tga.GPS, 1023, 17), (tga.GALILEO, 4092, 2),
+          (tga.GALILEO, 4092, 5), (tga.GALILEO, 4092, 16), (tga.L1C, 10230, 1), (tga.L1C, 10230, 5),
+          (tga.L1C, 10230, 16)]
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    with tga.Context(0) as c:
+        yield c
+
+
+def _rows(n_ant, n_bytes, seed):
+    return np.random.default_rng(seed).integers(0, 256, size=(n_ant, n_bytes), dtype=np.uint8)
+
+
+@pytest.mark.parametrize("precision", [tga.PRECISION_FP32, tga.PRECISION_FP16_TC])
+@pytest.mark.parametrize("const,chips,S", SHAPES)
+def test_few_rows_equal_many(ctx, const, chips, S, precision):
+    fs = 1.023e6 * S
+    bits = _rows(6, (2 * chips * S + 7) // 8 + 3, 10 * S)
+    prns = list(range(1, 27))
+    kw = dict(mask=1 << const, center_freq=0.3e6, search_band=400.0)
+    ctx.set_precision(precision)
+    try:
+        many = ctx.acquire_cells(bits, fs, prn_filter=prns, **kw)
+        few = ctx.acquire_cells(bits[:1], fs, prn_filter=[2], **kw)
+        two = ctx.acquire_cells(bits[:2], fs, prn_filter=[2, 5], **kw)
+    finally:
+        ctx.set_precision(tga.PRECISION_FP32)
+    sel = lambda r, a, p: [c for c in range(len(r)) if r["antenna"][c] == a and r["prn"][c] == p][0]
+    for r, cells in ((few, [(0, 2)]), (two, [(0, 2), (0, 5), (1, 2), (1, 5)])):
+        for a, p in cells:
+            for f in FIELDS:
+                assert r[f][sel(r, a, p)] == many[f][sel(many, a, p)], (f, a, p)
+
+
+@pytest.mark.parametrize("precision", [tga.PRECISION_FP32, tga.PRECISION_FP16_TC])
+@pytest.mark.parametrize("const,chips,S", SHAPES)
+def test_few_nc_rows_equal_many(ctx, const, chips, S, precision):
+    fs, blocks = 1.023e6 * S, 2
+    bits = _rows(6, (blocks * chips * S + 7) // 8 + 3, 11 * S)
+    kw = dict(center_freq=0.3e6, bin_step_hz=120.0, n_bins=3, blocks=blocks)
+    ctx.set_precision(precision)
+    try:
+        many = ctx.search_noncoherent(bits, fs, const, prns=list(range(1, 27)), **kw)
+        few = ctx.search_noncoherent(bits[:1], fs, const, prns=[2], **kw)
+    finally:
+        ctx.set_precision(tga.PRECISION_FP32)
+    at = [c for c in range(len(many)) if many["antenna"][c] == 0 and many["prn"][c] == 2][0]
+    for f in NC_FIELDS:
+        assert few[f][0] == many[f][at], f
+
+
+@pytest.mark.parametrize("n_bins", [1, 2, 15, 16, 17, 33])
+def test_bin_reduction_widths(ctx, n_bins):
+    """The reduction's choice against one search per bin."""
+    S, fs, step = 4, 4.092e6, 300.0
+    bits = _rows(3, 3 * 4092 // 8, n_bins)
+    kw = dict(prns=[1, 7, 32], bin_step_hz=step, blocks=2)
+    r = ctx.search_noncoherent(bits, fs, tga.GPS, center_freq=0.4e6, n_bins=n_bins, **kw)
+    each = [ctx.search_noncoherent(bits, fs, tga.GPS, center_freq=0.4e6 + (b - (n_bins - 1) // 2) * step, n_bins=1,
+                                   **kw) for b in range(n_bins)]
+    power = np.stack([e["power"] for e in each])
+    assert np.array_equal(r["power"], power.max(axis=0))
+    pick = n_bins - 1 - power[::-1].argmax(axis=0)  # the last of equal maxima
+    assert np.array_equal(r["best_freq_idx"], pick)
+    for f in ("best_codephase", "second_power"):
+        assert np.array_equal(r[f], np.stack([e[f] for e in each])[pick, np.arange(len(r))]), f
+
+
+@pytest.mark.parametrize("extra", [1, 3, 8, 15, 16, 1021])
+def test_rows_at_every_alignment(ctx, extra):
+    """17 rows of an odd (or even) number of bytes: starts at all offsets of a
+    16-byte word; the mean enters every sample."""
+    rng = np.random.default_rng(extra)
+    n = 2 * 1023 * 2 // 8 + 1 + extra
+    bits = rng.integers(0, 256, size=(17, n), dtype=np.uint8) | rng.integers(0, 256, size=(17, 1), dtype=np.uint8)
+    kw = dict(mask=1 << tga.GPS, prn_filter=[3], center_freq=0.3e6, search_band=400.0)
+    r = ctx.acquire_cells(bits, 2.046e6, **kw)
+    for a in range(17):
+        one = ctx.acquire_cells(bits[a:a + 1], 2.046e6, **kw)
+        for f in FIELDS:
+            assert one[f][0] == r[f][r["antenna"] == a][0], (a, f)
