@@ -98,3 +98,18 @@ def test_rows_at_every_alignment(ctx, extra):
         one = ctx.acquire_cells(bits[a:a + 1], 2.046e6, **kw)
         for f in FIELDS:
             assert one[f][0] == r[f][r["antenna"] == a][0], (a, f)
+
+
+@pytest.mark.parametrize("const,chips,S,band", [(tga.L1C, 10230, 1, 600.0), (tga.L1C, 10230, 3, 900.0),
+                                                (tga.GALILEO, 4092, 4, 2000.0)])
+def test_antenna_groups_share_phasors(ctx, const, chips, S, band):
+    """Seven antennas in groups that leave a shorter last one, each against a
+    search of that antenna alone."""
+    fs = 1.023e6 * S
+    bits = _rows(7, (2 * chips * S + 7) // 8 + 3, 12 * S)
+    kw = dict(mask=1 << const, prn_filter=[4], center_freq=0.3e6, search_band=band)
+    r = ctx.acquire_cells(bits, fs, **kw)
+    for a in range(7):
+        one = ctx.acquire_cells(bits[a:a + 1], fs, **kw)
+        for f in FIELDS:
+            assert one[f][0] == r[f][r["antenna"] == a][0], (a, f)
