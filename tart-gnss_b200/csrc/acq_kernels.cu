@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
   extern __shared__ float2 buf[];
   __shared__ unsigned long long s_key;
   __shared__ unsigned int s_p2;
+  __shared__ unsigned int s_floor;
   __shared__ bool s_last;
   // CAND with p2rows: for every residue of the row and every warp that
   // scanned it, its four largest |y|^2 as (value bits << 32) | lag, after
@@ -392,13 +393,17 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
       const int a = q2 % 31, rho = q2 / 31;
       return rho + S * G::natural(a, b, c);
     };
+    float pws[NC];
+    float floor_pw = -1.f;
     float pbest = 0.f;
     if (tid == 0) {
       s_key = 0ull;
       s_p2 = 0u;
+      s_floor = 0u;
     }
 
     for (int g = g0; g < g1; ++g) {
+      if (ARGMAX && NC > 1 && g > g0) floor_pw = fmaxf(floor_pw, __uint_as_float(s_floor));
       // sequence of slot s in this group, or -1 when idle
       auto seq_of = [&](int s) -> int {
         if (INV) {
@@ -407,6 +412,14 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
         }
         const int q = w * BC + s;
         return q < p.n_seq ? q : -1;
+      };
+      auto peak = [&](int code, float pw) {
+        if (pw == pmax) {
+          // exact tie: the reference keeps the later lag (Iterator::max_by)
+          if (lag_of(code) > lag_of(cmax)) cmax = code;
+        }
+        cmax = pw > pmax ? code : cmax;
+        pmax = fmaxf(pw, pmax);
       };
       // epilogue for output (s, a, b, c)
       auto epilogue = [&](int s, int a, int b, int c, float2 v) {
@@ -421,12 +434,10 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
           const float pw = fmaf(v.x, v.x, v.y * v.y);
           if (ARGMAX) {
             const int code = ((seq_of(s) * 31 + a) * 33 + b) * 16 + c;
-            if (pw == pmax) {
-              // exact tie: the reference keeps the later lag (Iterator::max_by)
-              if (lag_of(code) > lag_of(cmax)) cmax = code;
-            }
-            cmax = pw > pmax ? code : cmax;
-            pmax = fmaxf(pw, pmax);
+            if (NC == 1)
+              peak(code, pw);
+            else
+              pws[c] = pw;
             // kept in place for the second peak: the stage read its inputs
             // from these positions into registers before any output
             if (keep_top) reinterpret_cast<float*>(buf)[2 * (s * LC + G::offset(a, b, c))] = pw;
@@ -438,6 +449,21 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
             if (dist > p.chip_width) pbest = fmaxf(pbest, pw);
           }
         }
+      };
+
+      // CORR / CAND: the outputs of one DFT-M.  Only a value at or above the
+      // largest of the CTA's earlier groups can be the row's, so one comparison
+      // of their maximum does for nearly all of them (compares and selects per
+      // output took a tenth of the instructions: Lc = 10230 and 4092 take 4 %
+      // less time so; the 33 outputs of Lc = 1023 would cost registers, 8 % more)
+      auto peaks = [&](int s, int a, int b) {
+        float m = pws[0];
+#pragma unroll
+        for (int c = 1; c < NC; ++c) m = fmaxf(m, pws[c]);
+        if (m < floor_pw) return;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) peak(((seq_of(s) * 31 + a) * 33 + b) * 16 + c, pws[c]);
+        floor_pw = fmaxf(floor_pw, pmax);
       };
 
       // ---- stage 1: DFT-31 over digit a, input straight from global ----
@@ -508,7 +534,12 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
 #pragma unroll
           for (int c = 0; c < NC; ++c) x[c] = base[c * 33];
           dft_small<NC, INV>(x, [&](int tc, float2 v) { epilogue(s, a, b, tc, v); });
+          if (ARGMAX) peaks(s, a, b);
         }
+      }
+      if (ARGMAX && NC > 1 && g + 1 < g1) {
+        const unsigned mine = __reduce_max_sync(0xffffffffu, pmax > 0.f ? __float_as_uint(pmax) : 0u);
+        if ((tid & 31) == 0 && mine > s_floor) atomicMax(&s_floor, mine);
       }
       __syncthreads();
       // CAND with p2rows: the four largest |y|^2 of every residue of the

@@ -7,8 +7,13 @@
 //
 //  * odd prime R (3, 5, 11, 31): symmetric split into s_n = x_n + x_{R-n} and
 //    d_n = x_n - x_{R-n}; each output pair (k, R-k) costs (R-1) real FMAs per
-//    component, issued as packed FP32 pairs (re, im): 2*((R-1)/2)^2 + O(R)
-//    instructions per R points.
+//    component: 2*((R-1)/2)^2 + O(R) packed (re, im) instructions per R points,
+//    or twice as many scalar ones for R = 31.  A packed one takes two slots of
+//    the FMA pipe, so neither is faster by itself; in the correlator packed 3,
+//    5 and 11 leave issue slots to other warps (Lc = 10230 and 1023: 4 and 6 %
+//    less time), packed 31 costs registers (1 to 7 % more time).
+//    The non-coherent correlator's DFT-33 is faster unpacked (367 against 375 us
+//    for 32 PRNs x 21 bins x 10 periods).
 //  * 33 = 3 x 11 and 10 = 2 x 5 as Good-Thomas prime-factor maps (no twiddles):
 //    input digit map n = (N2*n1 + N1*n2) mod N, output map by the Chinese
 //    remainder theorem.
@@ -74,20 +79,8 @@ template <> __device__ __forceinline__ float kcos<11>(int m) { return kCos11[m];
 template <> __device__ __forceinline__ float ksin<11>(int m) { return kSin11[m]; }
 template <> __device__ __forceinline__ float kcos<31>(int m) { return kCos31[m]; }
 template <> __device__ __forceinline__ float ksin<31>(int m) { return kSin31[m]; }
-// the same constants as (v, v) pairs
-template <int R> __device__ __forceinline__ float2 kcos2(int m);
-template <int R> __device__ __forceinline__ float2 ksin2(int m);
-template <> __device__ __forceinline__ float2 kcos2<3>(int m) { return kCos3x2[m]; }
-template <> __device__ __forceinline__ float2 ksin2<3>(int m) { return kSin3x2[m]; }
-template <> __device__ __forceinline__ float2 kcos2<5>(int m) { return kCos5x2[m]; }
-template <> __device__ __forceinline__ float2 ksin2<5>(int m) { return kSin5x2[m]; }
-template <> __device__ __forceinline__ float2 kcos2<11>(int m) { return kCos11x2[m]; }
-template <> __device__ __forceinline__ float2 ksin2<11>(int m) { return kSin11x2[m]; }
-template <> __device__ __forceinline__ float2 kcos2<31>(int m) { return kCos31x2[m]; }
-template <> __device__ __forceinline__ float2 ksin2<31>(int m) { return kSin31x2[m]; }
-
 // DFT of odd prime length R; input x[0..R-1] (read only), outputs via st.
-template <int R, bool INV, class St>
+template <int R, bool INV, bool PACK = (R < 31), class St>
 __device__ __forceinline__ void dft_odd(const float2 (&x)[R], St&& st) {
   constexpr int H = (R - 1) / 2;
   float2 s[H], d[H];
@@ -109,10 +102,15 @@ __device__ __forceinline__ void dft_odd(const float2 (&x)[R], St&& st) {
     for (int n = 1; n <= H; ++n) {
       const int m = (n * k) % R;
       const float c = kcos<R>(m), sn = ksin<R>(m);
-      A.x = fmaf(s[n - 1].x, c, A.x);
-      A.y = fmaf(s[n - 1].y, c, A.y);
-      B.x = fmaf(d[n - 1].x, sn, B.x);
-      B.y = fmaf(d[n - 1].y, sn, B.y);
+      if constexpr (PACK) {
+        A = __ffma2_rn(s[n - 1], make_float2(c, c), A);
+        B = __ffma2_rn(d[n - 1], make_float2(sn, sn), B);
+      } else {
+        A.x = fmaf(s[n - 1].x, c, A.x);
+        A.y = fmaf(s[n - 1].y, c, A.y);
+        B.x = fmaf(d[n - 1].x, sn, B.x);
+        B.y = fmaf(d[n - 1].y, sn, B.y);
+      }
     }
     // forward: X[k] = A - iB, X[R-k] = A + iB; inverse swaps them.
     const float2 lo = make_float2(A.x + B.y, A.y - B.x);
@@ -128,17 +126,17 @@ __device__ __forceinline__ void dft_odd(const float2 (&x)[R], St&& st) {
 }
 
 // 33 = 3 x 11.  Input digits: n = (11 n1 + 3 n2) mod 33; output k = (22 k1 + 12 k2) mod 33.
-template <bool INV, class St>
+template <bool INV, bool PACK = true, class St>
 __device__ __forceinline__ void dft33(const float2 (&x)[33], St&& st) {
   float2 u[3][11];
 #pragma unroll
   for (int n2 = 0; n2 < 11; ++n2) {
     const float2 t[3] = {x[(3 * n2) % 33], x[(11 + 3 * n2) % 33], x[(22 + 3 * n2) % 33]};
-    dft_odd<3, INV>(t, [&](int k1, float2 v) { u[k1][n2] = v; });
+    dft_odd<3, INV, PACK>(t, [&](int k1, float2 v) { u[k1][n2] = v; });
   }
 #pragma unroll
   for (int k1 = 0; k1 < 3; ++k1) {
-    dft_odd<11, INV>(u[k1], [&](int k2, float2 v) { st((22 * k1 + 12 * k2) % 33, v); });
+    dft_odd<11, INV, PACK>(u[k1], [&](int k2, float2 v) { st((22 * k1 + 12 * k2) % 33, v); });
   }
 }
 

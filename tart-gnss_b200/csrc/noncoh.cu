@@ -283,9 +283,9 @@ __global__ void __launch_bounds__(NT, MINB) nc_correlate_kernel(NcParams p) {
 #pragma unroll
           for (int b = 0; b < 33; ++b) x[b] = base[b];
           if constexpr (NC == 1) {
-            dft33<true>(x, [&](int tb, float2 v) { accumulate(s, a, tb, 0, v); });
+            dft33<true, false>(x, [&](int tb, float2 v) { accumulate(s, a, tb, 0, v); });
           } else {
-            dft33<true>(x, [&](int tb, float2 v) { base[tb] = v; });
+            dft33<true, false>(x, [&](int tb, float2 v) { base[tb] = v; });
           }
         }
         // stage 3: DFT-M over digit c

@@ -113,3 +113,17 @@ def test_antenna_groups_share_phasors(ctx, const, chips, S, band):
         one = ctx.acquire_cells(bits[a:a + 1], fs, **kw)
         for f in FIELDS:
             assert one[f][0] == r[f][r["antenna"] == a][0], (a, f)
+
+
+@pytest.mark.parametrize("n_ant,n_prn", [(1, 1), (6, 26)])
+@pytest.mark.parametrize("const,chips,S", [(tga.GPS, 1023, 9), (tga.GALILEO, 4092, 5), (tga.L1C, 10230, 3)])
+def test_all_equal_takes_the_last(ctx, const, chips, S, n_ant, n_prn):
+    """A constant recording has no signal left after its mean: every value is
+    0, and of equal values the last lag and the last bin are taken."""
+    P, fs = chips * S, 1.023e6 * S
+    bits = np.full((n_ant, (2 * P + 7) // 8), 255, dtype=np.uint8)
+    r = ctx.acquire_cells(bits, fs, mask=1 << const, prn_filter=list(range(1, n_prn + 1)), center_freq=0.3e6,
+                          search_band=600.0)
+    assert len(r) == n_ant * n_prn
+    assert np.all(r["best_codephase"] == P - 1)
+    assert np.all(r["best_freq_idx"] == 4) and np.all(r["hypothesis"] == 0)
