@@ -127,3 +127,23 @@ def test_all_equal_takes_the_last(ctx, const, chips, S, n_ant, n_prn):
     assert len(r) == n_ant * n_prn
     assert np.all(r["best_codephase"] == P - 1)
     assert np.all(r["best_freq_idx"] == 4) and np.all(r["hypothesis"] == 0)
+
+
+@pytest.mark.parametrize("precision", [tga.PRECISION_FP32, tga.PRECISION_FP16_TC])
+@pytest.mark.parametrize("const,chips,S", [(tga.GPS, 1023, 1), (tga.GPS, 1023, 9), (tga.GALILEO, 4092, 3),
+                                           (tga.L1C, 10230, 1), (tga.L1C, 10230, 3)])
+def test_odd_numbers_of_sequences(ctx, const, chips, S, precision):
+    """One antenna, bin and block: S sequences, the last of them alone in its
+    forward transform; against the same cell among three antennas."""
+    fs = 1.023e6 * S
+    bits = _rows(3, (chips * S + 7) // 8 + 2, 13 * S)
+    kw = dict(bin_step_hz=200.0, blocks=1)
+    ctx.set_precision(precision)
+    try:
+        one = ctx.search_noncoherent(bits[1:2], fs, const, prns=[3], center_freq=0.3e6, n_bins=1, **kw)
+        many = ctx.search_noncoherent(bits, fs, const, prns=[3], center_freq=0.3e6, n_bins=1, **kw)
+    finally:
+        ctx.set_precision(tga.PRECISION_FP32)
+    at = [c for c in range(len(many)) if many["antenna"][c] == 1][0]
+    for f in NC_FIELDS:
+        assert one[f][0] == many[f][at], f
