@@ -190,16 +190,6 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(p));
   return p != 0;
 }
-// 16 columns of the warp's 32 lanes, one lane per thread
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
-      "[%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
 // 16 columns of 16 lanes: thread t gets, for i = 0 .. 3, column 4 i + t % 4 of
 // lane t / 4 in r[2 i] and of lane t / 4 + 8 in r[2 i + 1]
 __device__ __forceinline__ void tmem_ld_pairs(uint32_t taddr, uint32_t (&r)[8]) {
@@ -228,7 +218,6 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[4]) {
                : "memory");
 }
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld8(taddr, r); }
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
 __device__ __forceinline__ void tmem_st_zero8(uint32_t taddr) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(0u)
                : "memory");
@@ -470,15 +459,41 @@ struct TcParams {
   // work units: item u / split, rounds [r0, r1) of part u % split; a round is
   // one PRN (NCB: a pair of PRNs, one per chain)
   int split;
+  int step_w, step_r;  // NCB: gridDim.x units on, in items and rounds
   int n_rounds, n_prn, S;
   int B;            // coherent blocks summed non-coherently (1: the drop-in search)
   int skip_commit;  // test hook: see TGA_TEST_TC_SKIP_COMMIT
 };
 
-__device__ __forceinline__ int unit_round0(int split, int u, int n) { return (int)((long long)(u % split) * n / split); }
-__device__ __forceinline__ int unit_round1(int split, int u, int n) {
-  return (int)((long long)(u % split + 1) * n / split);
-}
+// The CTA's units in order: item w, rounds [r0, r1).
+template <bool NCB>
+struct Units {
+  const TcParams& p;
+  int u, w, r0, r1;
+  __device__ __forceinline__ explicit Units(const TcParams& q) : p(q), u(blockIdx.x) {
+    w = u / p.split;
+    set(u - w * p.split);
+  }
+  __device__ __forceinline__ bool more() const { return w < p.n_items; }
+  __device__ __forceinline__ void next() {
+    if (NCB) {  // one round per unit: no division per round
+      r0 += p.step_r;
+      w += p.step_w;
+      if (r0 >= p.split) r0 -= p.split, ++w;
+      r1 = r0 + 1;
+    } else {
+      u += gridDim.x;
+      w = u / p.split;
+      set(u - w * p.split);
+    }
+  }
+
+ private:
+  __device__ __forceinline__ void set(int part) {
+    r0 = NCB ? part : (int)((long long)part * p.n_rounds / p.split);
+    r1 = NCB ? part + 1 : (int)((long long)(part + 1) * p.n_rounds / p.split);
+  }
+};
 
 // mbarriers of the CTA and who completes them.  Step s is chain s % NCH's use
 // s / NCH; a barrier of a chain is in phase (s / NCH) & 1.
@@ -505,17 +520,14 @@ __device__ __forceinline__ bool m1_role(const TcParams& p, uint32_t bars, uint32
                                         uint32_t tmem) {
   using T = Tc<M, NCB>;
   using Br = Bars<T>;
-  const int n_units = p.n_items * p.split, B = NCB ? p.B : 1;
+  const int B = NCB ? p.B : 1;
   constexpr int PER_ROUND = NCB ? 2 : 1;  // code blocks of a round
   // ---- code blocks in order: block `fetched` is chain fx of round fr of unit fu ----
-  int fu = blockIdx.x, fr = 0, fr1 = 0, fx = 0, fetched = 0;
-  if (fu < n_units) {
-    fr = unit_round0(p.split, fu, p.n_rounds);
-    fr1 = unit_round1(p.split, fu, p.n_rounds);
-  }
+  Units<NCB> fu(p);
+  int fr = fu.r0, fx = 0, fetched = 0;
   auto fetch = [&]() {
-    if (fu >= n_units) return;
-    const int hyp = NCB ? 0 : (fu / p.split / p.groups) & 1;
+    if (!fu.more()) return;
+    const int hyp = NCB ? 0 : (fu.w / p.groups) & 1;
     int prn = NCB ? 2 * fr + fx : fr;
     if (prn >= p.n_prn) prn = p.n_prn - 1;  // an odd PRN number: the last one on both chains
     const int slot = fetched % T::SLOTS;
@@ -525,10 +537,9 @@ __device__ __forceinline__ bool m1_role(const TcParams& p, uint32_t bars, uint32
     ++fetched;
     if (++fx == PER_ROUND) {
       fx = 0;
-      if (++fr == fr1) {
-        fu += gridDim.x;
-        fr = unit_round0(p.split, fu, p.n_rounds);
-        fr1 = unit_round1(p.split, fu, p.n_rounds);
+      if (++fr == fu.r1) {
+        fu.next();
+        fr = fu.r0;
       }
     }
   };
@@ -538,8 +549,7 @@ __device__ __forceinline__ bool m1_role(const TcParams& p, uint32_t bars, uint32
   auto issue = [&](auto xc) {
     constexpr int x = decltype(xc)::value;
 #pragma unroll
-    for (int ks = 0; ks < T::K1 / 16; ++ks)
-{
+    for (int ks = 0; ks < T::K1 / 16; ++ks) {
       const uint64_t dbk = db + (uint64_t)(x * (T::B_BYTES >> 4) + ks * (256 >> 4));
       if (ks < T::A1_KS)
         mma_f16_ta(tmem + (uint32_t)(x * T::N1), tmem + (uint32_t)(T::A1_COL + 8 * ks), dbk, idesc_f16(T::N1, true),
@@ -552,8 +562,8 @@ __device__ __forceinline__ bool m1_role(const TcParams& p, uint32_t bars, uint32
   };
   int s = 0, commits = 0;
   bool ok = bounded_wait(bars + Br::A1, 0u) != 0;
-  for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-    const int n = (unit_round1(p.split, u, p.n_rounds) - unit_round0(p.split, u, p.n_rounds)) * PER_ROUND * B;
+  for (Units<NCB> u(p); u.more() && ok; u.next()) {
+    const int n = (u.r1 - u.r0) * PER_ROUND * B;
     int left = NCB ? PER_ROUND * B : 1;  // steps of the round (of its code blocks) from here on
 #pragma unroll 1
     for (int i = 0; i < n; ++i, ++s) {
@@ -607,7 +617,7 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
   const uint32_t ZS = CODE + T::SLOTS * T::CODE_REGION;
   const uint32_t bars = smem_addr(s_bar);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const int S = p.S, split = p.split, B = NCB ? p.B : 1, n_units = p.n_items * split;
+  const int S = p.S, B = NCB ? p.B : 1;
 
   if (warp == 0) {
     tmem_alloc(&s_tmem, kTcTmemCols);
@@ -821,9 +831,9 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
     };
     uint32_t use = 0;  // of the chain
     int s = 0;         // chain of the next step (drop-in search: steps run on across units)
-    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-      const int ab_h = u / split / p.groups, r1 = unit_round1(split, u, p.n_rounds);
-      for (int r = unit_round0(split, u, p.n_rounds); r < r1 && ok; ++r) {
+    for (Units<NCB> u(p); u.more() && ok; u.next()) {
+      const int ab_h = u.w / p.groups;
+      for (int r = u.r0; r < u.r1 && ok; ++r) {
         if (!NCB) {
           const bool mine = s == x;
           s = s + 1 == T::NCH ? 0 : s + 1;
@@ -950,16 +960,16 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
       return true;
     };
     int s = 0, n = 0;
-    if ((int)blockIdx.x < n_units) load_z(blockIdx.x / split, 0);
-    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-      const int w = u / split, r1 = unit_round1(split, u, p.n_rounds);
-      for (int r = unit_round0(split, u, p.n_rounds); r < r1 && ok; ++r) {
+    Units<NCB> u(p);
+    if (u.more()) load_z(u.w, 0);
+    while (u.more() && ok) {
+      for (int r = u.r0; r < u.r1 && ok; ++r) {
         if constexpr (NCB) {
 #pragma unroll 1
           for (int blk = 0; blk < B && ok; ++blk, s += 2) {
             ok = products(s, n, blk == 0) && products(s + 1, n + 1, blk == 0);
             // the next block's Z, while the products' buffers are in use
-            if (blk + 1 < B || r + 1 < r1) load_z(w, blk + 1 < B ? blk + 1 : 0);
+            if (blk + 1 < B) load_z(u.w, blk + 1);
           }
           n += 2;
         } else {
@@ -968,7 +978,8 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
           ++n;
         }
       }
-      if (u + (int)gridDim.x < n_units) load_z((u + gridDim.x) / split, 0);
+      u.next();
+      if (u.more()) load_z(u.w, 0);
     }
   } else {
     if (elect_one()) ok = m1_role<M, NCB>(p, bars, A1, PROD, CODE, tmem);
@@ -1000,11 +1011,26 @@ cudaError_t run_tc(const PolyClass& pc, const SearchDims& dims, int B, const voi
   p.n_items = dims.n_ant * dims.nb * (NCB ? 1 : 2) * p.groups;
   if (p.n_items < 1 || p.n_prn < 1) return cudaSuccess;
   p.n_rounds = NCB ? (p.n_prn + 1) / 2 : p.n_prn;
-  // too few items to fill the SMs: split each item's rounds over CTAs
-  p.split = 1;
-  if (p.n_items < num_sms) {
-    p.split = (num_sms + p.n_items - 1) / p.n_items;
-    if (p.split > p.n_rounds) p.split = p.n_rounds;
+  // Non-coherent: a unit is one round, so the CTAs take neighbouring rounds at
+  // any time and share an item's Z (read for every round) in L2, and no CTA has
+  // more than one round more than another.  Whole items, split only when there
+  // were fewer than SMs, left up to 43 % of the SMs idle in a last pass (one
+  // antenna, 21 bins, 100 blocks: 8.2 -> 4.5 ms at Lc = 1023, 9.0 -> 7.4 at 4092,
+  // 45.1 -> 43.2 at 10230, which the power limit holds by then).
+  // Drop-in: Z is read once per unit, so as few parts as the SMs' shares allow:
+  // a unit costs its rounds and about two more to change Z.
+  // One antenna, 41 bins: 186 -> 154 us at Lc = 1023, 285 -> 264 at 4092.
+  p.split = p.n_rounds;
+  if (!NCB) {
+    double best = 0.0;
+    for (int split = 1; split <= 32 && split <= p.n_rounds; ++split) {
+      const long long per_sm = ((long long)p.n_items * split + num_sms - 1) / num_sms;
+      const double cost = (double)per_sm * ((p.n_rounds + split - 1) / split + 2.0);
+      if (split == 1 || cost < best) {
+        best = cost;
+        p.split = split;
+      }
+    }
   }
   auto kern = pfa_tc_kernel<M, NCB>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
@@ -1013,6 +1039,8 @@ cudaError_t run_tc(const PolyClass& pc, const SearchDims& dims, int B, const voi
   // 512-column TMEM allocation never meets another one
   int grid = num_sms;
   if (grid > p.n_items * p.split) grid = p.n_items * p.split;
+  p.step_w = grid / p.split;
+  p.step_r = grid % p.split;
   kern<<<grid, T::THREADS, T::SMEM, st>>>(p);
   kernel_launch_add(1);
   return cudaGetLastError();

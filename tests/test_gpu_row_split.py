@@ -147,3 +147,27 @@ def test_odd_numbers_of_sequences(ctx, const, chips, S, precision):
     at = [c for c in range(len(many)) if many["antenna"][c] == 1][0]
     for f in NC_FIELDS:
         assert one[f][0] == many[f][at], f
+
+
+@pytest.mark.parametrize("const,chips,S,n_prn,n_bins", [(tga.GPS, 1023, 9, 32, 33), (tga.GALILEO, 4092, 3, 50, 33),
+                                                        (tga.GALILEO, 4092, 6, 7, 51), (tga.L1C, 10230, 2, 63, 33)])
+def test_tensor_core_shares(ctx, const, chips, S, n_prn, n_bins):
+    """Numbers of items between one and three times the SMs, whose rounds are
+    divided: the FP32 cells, drop-in and non-coherent."""
+    fs = 1.023e6 * S
+    bits = _rows(1, (3 * chips * S + 7) // 8 + 2, 14 * S)
+    prns = list(range(1, n_prn + 1))
+    a, b = [], []
+    for out, precision in ((a, tga.PRECISION_FP32), (b, tga.PRECISION_FP16_TC)):
+        ctx.set_precision(precision)
+        try:
+            out.append(ctx.acquire_cells(bits, fs, mask=1 << const, prn_filter=prns, center_freq=0.3e6,
+                                         search_band=150.0 * (n_bins - 1)))
+            out.append(ctx.search_noncoherent(bits, fs, const, prns=prns, center_freq=0.3e6, bin_step_hz=150.0,
+                                              n_bins=n_bins, blocks=3))
+        finally:
+            ctx.set_precision(tga.PRECISION_FP32)
+    for f in FIELDS:
+        assert np.array_equal(a[0][f], b[0][f]), f
+    for f in NC_FIELDS:
+        assert np.array_equal(a[1][f], b[1][f]), f
