@@ -490,8 +490,8 @@ struct Units {
 
  private:
   __device__ __forceinline__ void set(int part) {
-    r0 = NCB ? part : (int)((long long)part * p.n_rounds / p.split);
-    r1 = NCB ? part + 1 : (int)((long long)(part + 1) * p.n_rounds / p.split);
+    r0 = NCB ? part : part * p.n_rounds / p.split;  // (split <= 32)
+    r1 = NCB ? part + 1 : (part + 1) * p.n_rounds / p.split;
   }
 };
 
