@@ -49,6 +49,14 @@ struct tga_ctx {
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t copied[2] = {nullptr, nullptr};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  // tga_acquire_all: streams of the code classes after the first, forked from
+  // `stream` at `forked` and joined at each one's `joined` (created on first use)
+  struct Side {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t joined = nullptr;
+  };
+  std::vector<Side> sides;
+  cudaEvent_t forked = nullptr;
   std::string err;
   std::map<std::string, DevBuf> bufs;
   // cached fused-path code spectra: key -> (device D, n_prn)
@@ -548,13 +556,26 @@ GroupBufs prepare_group(tga_ctx* ctx, const ClassGroup& grp, int n_ant, int nb, 
 // Enqueues the fused pipeline of one class group on the context stream
 // (launches, memsets and the copy of the finalised cells into host_out,
 // pinned memory of n_ant * n_prn CellOut).
+// The part of a class's search that needs no signal.
+void enqueue_codes(tga_ctx* ctx, const ClassGroup& grp, const GroupBufs& b, cudaStream_t st) {
+  const PolyClass& pc = grp.pc;
+  const int n_prn = (int)grp.prns.size();
+  const std::string cls = "[Lc=" + std::to_string(pc.Lc) + "]";
+  timed(ctx, ("code_spectra" + cls).c_str(), (double)n_prn * 2 * fft_flops(pc.Lc),
+        [&] { return launch_code_spectra(pc, b.chips, n_prn, b.D, ctx->num_sms, st); });
+  if (ctx->precision == TGA_PRECISION_FP16_TC)
+    timed(ctx, ("tc_pack" + cls).c_str(), 0.0,
+          [&] { return launch_tc_pack(pc, b.D, (long long)n_prn * 2, true, b.d16, ctx->num_sms, st); });
+}
+
+// The rest of it, after enqueue_codes (and in tensor-core mode after *b.err is 0).
 void enqueue_group(tga_ctx* ctx, const ClassGroup& grp, const GroupBufs& b, const SampleSource& src,
-                   const double* d_fc, int nb, double center, int want_cn0, int chip_width, CellOut* host_out) {
+                   const double* d_fc, int nb, double center, int want_cn0, int chip_width, CellOut* host_out,
+                   cudaStream_t st) {
   const PolyClass& pc = grp.pc;
   const int n_ant = src.n_ant;
   const int n_prn = (int)grp.prns.size();
   const int n_ab = n_ant * nb;
-  cudaStream_t st = ctx->stream;
 
   SearchDims dims;
   dims.n_ant = n_ant;
@@ -569,19 +590,13 @@ void enqueue_group(tga_ctx* ctx, const ClassGroup& grp, const GroupBufs& b, cons
   // while at most three lags of a residue lie within chip_width of the peak
   // (chip_width = S samples at every fused rate)
   const bool rows_p2 = ctx->precision == TGA_PRECISION_FP16_TC && (2 * chip_width + pc.S) / pc.S <= 3;
-  timed(ctx, ("code_spectra" + cls).c_str(), (double)n_prn * 2 * fft_flops(pc.Lc),
-        [&] { return launch_code_spectra(pc, b.chips, n_prn, b.D, ctx->num_sms, st); });
   timed(ctx, ("frontend" + cls).c_str(), (double)n_ab * 10.0 * pc.P,
         [&] { return launch_frontend(src, dims, pc, b.z, st); });
   if (ctx->precision == TGA_PRECISION_FP16_TC) {
-    // the forward transform also writes Z's FP16 operands; the code spectra
-    // are packed apart
+    // the forward transform also writes Z's FP16 operands
     timed(ctx, ("forward_z" + cls).c_str(), (double)n_ab * 2 * fft_flops(pc.P), [&] {
       return launch_forward_z_tc(pc, n_ab, b.z, b.z16, b.zmap, tc_z_scale(pc), ctx->num_sms, st);
     });
-    timed(ctx, ("tc_pack" + cls).c_str(), 0.0,
-          [&] { return launch_tc_pack(pc, b.D, (long long)n_prn * 2, true, b.d16, ctx->num_sms, st); });
-    CK(cudaMemsetAsync(b.err, 0, sizeof(int), st));
     CK(cudaMemsetAsync(b.keys, 0, (size_t)n_ab * 2 * n_prn * sizeof(unsigned long long), st));
     timed(ctx, ("correlate_tc" + cls).c_str(), (double)n_ab * 2 * n_prn * row, [&] {
       return launch_correlate_tc(pc, dims, b.bmat, b.z16, b.d16, b.keys, b.err, ctx->test_flags, ctx->num_sms, st);
@@ -752,10 +767,35 @@ int acquire_all_impl(tga_ctx* ctx, const uint8_t* d_bits, size_t n_ant_total, si
     // antenna means over the whole rows
     timed(ctx, "antenna_means", 0.0,
           [&] { return launch_antenna_means(d_bits, (int)n_ant_total, row_bytes, d_mean, st); });
-    for (size_t gi = 0; gi < groups.size(); ++gi)
+    if (ctx->precision == TGA_PRECISION_FP16_TC && !gbufs.empty()) CK(cudaMemsetAsync(gbufs[0].err, 0, sizeof(int), st));
+    // The classes share no buffer that one of them writes, apart from the error
+    // flag they may all set.  In a short search a stream each lets the small
+    // kernels of one class run beside the others' (one antenna, tensor cores:
+    // 2.81 -> 2.66 ms; a few antennas and PRNs in FP32: 3.08 -> 2.98 ms).  In a
+    // long one the correlators of two lengths would share SMs and their
+    // instruction caches (24 antennas in FP32: 179.9 -> 185.2 ms, 57.1 -> 57.6 with
+    // tensor cores), so it keeps one, as per-kernel timing does.
+    double lags = 0.0;
+    for (const auto& g : groups) lags += (double)ants.size() * nb * (double)g.prns.size() * g.pc.P;
+    const bool fork = groups.size() > 1 && !ctx->profiling &&
+                      lags < (ctx->precision == TGA_PRECISION_FP16_TC ? 4e9 : 6e8);
+    if (fork) CK(cudaEventRecord(ctx->forked, st));
+    for (size_t gi = 0; gi < groups.size(); ++gi) {
+      const cudaStream_t gs = fork && gi > 0 ? ctx->sides[gi - 1].stream : st;
+      if (gs != st) CK(cudaStreamWaitEvent(gs, ctx->forked, 0));
+      enqueue_codes(ctx, groups[gi], gbufs[gi], gs);
       enqueue_group(ctx, groups[gi], gbufs[gi], src, d_fc, nb, opt->center_freq, opt->cn0, chip_width_of(fs),
-                    gout[gi]);
+                    gout[gi], gs);
+      if (gs != st) CK(cudaEventRecord(ctx->sides[gi - 1].joined, gs));
+    }
+    for (size_t gi = 1; fork && gi < groups.size(); ++gi) CK(cudaStreamWaitEvent(st, ctx->sides[gi - 1].joined, 0));
   };
+  if (groups.size() > 1 && !ctx->forked) CK(cudaEventCreateWithFlags(&ctx->forked, cudaEventDisableTiming));
+  while (ctx->sides.size() + 1 < groups.size()) {
+    ctx->sides.emplace_back();  // (in the list before it is filled: freed with the context)
+    CK(cudaStreamCreateWithFlags(&ctx->sides.back().stream, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&ctx->sides.back().joined, cudaEventDisableTiming));
+  }
   CK(cudaEventRecord(ctx->ev0, st));
   if (generic_consts.empty()) {
     // the plan: everything the launches take by value or by address
@@ -963,11 +1003,21 @@ int acquire_single_impl(tga_ctx* ctx, int c, const float* h_sig, const double* h
   cudaStream_t st = ctx->stream;
   float* d_sig = (float*)ctx->buf("single.sig", n * sizeof(float));
   double* d_pp = (double*)ctx->buf("single.pp", n * sizeof(double));
+  // the code spectra are computed while the host hands the signal over
+  ClassGroup g;
+  GroupBufs gb;
+  if (fused) {
+    g.pc = pc;
+    g.consts.push_back(c);
+    g.prns.push_back({c, prn});
+    gb = prepare_group(ctx, g, 1, nb, "single");
+    if (ctx->precision == TGA_PRECISION_FP16_TC) CK(cudaMemsetAsync(gb.err, 0, sizeof(int), st));
+    enqueue_codes(ctx, g, gb, st);
+  }
   CK(cudaMemcpyAsync(d_sig, h_sig, n * sizeof(float), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_pp, h_pp, n * sizeof(double), cudaMemcpyHostToDevice, st));
-  int32_t zero = 0;
   int32_t* d_ant = (int32_t*)ctx->buf("single.ant", sizeof(int32_t));
-  CK(cudaMemcpyAsync(d_ant, &zero, sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  CK(cudaMemsetAsync(d_ant, 0, sizeof(int32_t), st));
   double* d_fc = (double*)ctx->buf("single.fc", fc.size() * sizeof(double));
   CK(cudaMemcpyAsync(d_fc, fc.data(), fc.size() * sizeof(double), cudaMemcpyHostToDevice, st));
   if (!fused) {
@@ -983,14 +1033,9 @@ int acquire_single_impl(tga_ctx* ctx, int c, const float* h_sig, const double* h
   src.n_samples = n;
   src.ant = d_ant;
   src.n_ant = 1;
-  ClassGroup g;
-  g.pc = pc;
-  g.consts.push_back(c);
-  g.prns.push_back({c, prn});
   ctx->h2d += n * (sizeof(float) + sizeof(double));
-  const GroupBufs gb = prepare_group(ctx, g, 1, nb, "single");
   CellOut* cell = (CellOut*)ctx->host_pinned(sizeof(CellOut));
-  enqueue_group(ctx, g, gb, src, d_fc, nb, center, 0, chip_width_of(fs), cell);
+  enqueue_group(ctx, g, gb, src, d_fc, nb, center, 0, chip_width_of(fs), cell, st);
   CK(cudaStreamSynchronize(st));
   ctx->last_launches = kernel_launch_count();
   collect_times(ctx);
@@ -1076,6 +1121,11 @@ int tga_destroy(tga_ctx* ctx) {
   for (auto& kv : ctx->bufs)
     if (kv.second.p) cudaFree(kv.second.p);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+  for (tga_ctx::Side& sd : ctx->sides) {
+    if (sd.joined) cudaEventDestroy(sd.joined);
+    if (sd.stream) cudaStreamDestroy(sd.stream);
+  }
+  if (ctx->forked) cudaEventDestroy(ctx->forked);
   for (cudaEvent_t& e : ctx->copied)
     if (e) cudaEventDestroy(e);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
