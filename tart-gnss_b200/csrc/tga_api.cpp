@@ -980,7 +980,7 @@ tga_result generic_one(tga_ctx* ctx, int c, const float* d_sig, const double* d_
   const size_t cp = (size_t)ri[1] % period;
   r.best_codephase = (int64_t)cp;
   r.signal_strength = (double)rf[0];
-  r.second_peak = (double)rf[1];
+  r.second_peak = (double)(rf[1] > 0.f ? rf[1] : 1e-6f);  // 0 also without a candidate (correlate.rs:173-175)
   r.codephase_frac = (double)cp / (double)period;
   r.frequency = fc[ri[0]] - center;
   r.hypothesis = ri[2];
