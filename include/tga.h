@@ -121,7 +121,7 @@ const char* tga_version(void);
  * points), same AcquisitionResult.  When num_samples == 2 * samples_per_chunk
  * and the resampled code is a whole number of samples per chip the fused
  * polyphase kernels run; any other length runs the generic GPU path
- * (Bluestein FFTs of length num_samples). */
+ * (FFTs of length num_samples, of any length). */
 int tga_acquire_single(tga_ctx* ctx, int constellation, const float* h_signal_f32,
                        const double* h_phasepoints, size_t num_samples, double sampling_freq,
                        double center_freq, double search_band, int prn,
