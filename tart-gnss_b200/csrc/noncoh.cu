@@ -232,9 +232,7 @@ __global__ void __launch_bounds__(NT, MINB) nc_correlate_kernel(NcParams p) {
   unsigned long long* s_res = reinterpret_cast<unsigned long long*>(acc + BC * LC);
   const int tid = threadIdx.x, S = p.S;
   const int groups = (S + BC - 1) / BC;
-  // a row's residue groups are shared between CTAs as in pfa_kernel (32 rows
-  // of two groups: 97 us for the second peaks of 32 PRNs over ten periods on
-  // 32 CTAs, half on 64)
+  // a row's residue groups are shared between CTAs as in pfa_kernel
   const int rows = MODE == NC_CAND ? min(p.n_items, *p.cand_count) : p.n_items;
   const int split = MODE == NC_CAND ? (rows > 0 ? max(1, min(groups, (int)gridDim.x / rows)) : 1) : p.split;
   for (int unit = blockIdx.x; unit < rows * split; unit += gridDim.x) {
@@ -445,24 +443,35 @@ __global__ void __launch_bounds__(NT, MINB) nc_correlate_kernel(NcParams p) {
 
 // Two CTAs per SM hide each other's barriers where the buffers allow it
 // (32 PRNs x 21 bins x 10 periods of Lc = 1023: 455 us with one, 367 with two).
-template <int M>
+// FEW: fewer residues per CTA for calls whose rows' groups would not give every
+// SM a CTA: a block then takes its stages' latency, not the issue slots of nine
+// warps (second peaks of 32 PRNs over ten periods: 56 us on 64 CTAs, 37 on 256).
+template <int M, bool FEW>
 struct NcCfg;
 template <>
-struct NcCfg<1> {
+struct NcCfg<1, false> {
   static constexpr int BC = 8, NT = 288, MINB = 2;
 };
 template <>
-struct NcCfg<4> {
+struct NcCfg<1, true> {
+  static constexpr int BC = 2, NT = 96, MINB = 5;
+};
+template <>
+struct NcCfg<4, false> {
   static constexpr int BC = 2, NT = 288, MINB = 2;
 };
 template <>
-struct NcCfg<10> {
+struct NcCfg<4, true> {
+  static constexpr int BC = 1, NT = 160, MINB = 3;
+};
+template <>
+struct NcCfg<10, false> {
   static constexpr int BC = 1, NT = 352, MINB = 1;
 };
 
-template <int M, int MODE>
+template <int M, int MODE, bool FEW>
 cudaError_t run_nc(const NcParams& p, int num_sms, cudaStream_t st) {
-  using C = NcCfg<M>;
+  using C = NcCfg<M, FEW>;
   constexpr int LC = Geo<M>::LC;
   size_t smem = (size_t)C::BC * LC * (sizeof(float2) + sizeof(float));
   if (MODE == NC_CAND && p.p2rows) {
@@ -494,12 +503,21 @@ cudaError_t run_nc(const NcParams& p, int num_sms, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+template <int M, int MODE>
+cudaError_t pick_nc(const NcParams& p, int num_sms, cudaStream_t st) {
+  if constexpr (M != 10 && MODE != NC_CAND) {  // (a list's length is known on the device only)
+    const int groups = (p.S + NcCfg<M, false>::BC - 1) / NcCfg<M, false>::BC;
+    if ((long long)p.n_items * groups < num_sms) return run_nc<M, MODE, true>(p, num_sms, st);
+  }
+  return run_nc<M, MODE, false>(p, num_sms, st);
+}
+
 template <int MODE>
 cudaError_t dispatch_nc(int M, const NcParams& p, int num_sms, cudaStream_t st) {
   switch (M) {
-    case 1: return run_nc<1, MODE>(p, num_sms, st);
-    case 4: return run_nc<4, MODE>(p, num_sms, st);
-    case 10: return run_nc<10, MODE>(p, num_sms, st);
+    case 1: return pick_nc<1, MODE>(p, num_sms, st);
+    case 4: return pick_nc<4, MODE>(p, num_sms, st);
+    case 10: return pick_nc<10, MODE>(p, num_sms, st);
   }
   return cudaErrorInvalidValue;
 }
