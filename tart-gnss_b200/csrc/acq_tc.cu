@@ -56,9 +56,9 @@
 // cycles; 686 for M1, 432 for M2); the FP32 pipe about 900 (DFT-2, DFT-3 and
 // |y|^2: 8 operations per point).  Long runs sit at the 1000 W power limit.
 // Measured against the three-stage design before it, which transposed through
-// shared memory twice (24 antennas, 41 bins, --all): 62.2 -> 34.5 ms at Lc =
-// 10230, 11.2 -> 6.3 at 4092, 3.65 -> 3.55 at 1023; non-coherent, one antenna,
-// 100 ms: 81.1 -> 44.5, 16.6 -> 9.4 and 10.4 -> 8.4 ms; weak signals (24
+// shared memory twice (24 antennas, 41 bins, --all): 62.2 -> 35.3 ms at Lc =
+// 10230, 11.2 -> 6.1 at 4092, 3.65 -> 3.4 at 1023; non-coherent, one antenna,
+// 100 ms: 81.1 -> 43.2, 16.6 -> 7.4 and 10.4 -> 4.5 ms; weak signals (24
 // antennas, 201 bins, 10 blocks) 44.0 -> 28.8 ms.  RMS error of the FP16 row
 // keys 8.8e-5 -> 6.9e-5 of the largest row (one rounding of the data less).
 //
