@@ -780,15 +780,22 @@ int acquire_all_impl(tga_ctx* ctx, const uint8_t* d_bits, size_t n_ant_total, si
     const bool fork = groups.size() > 1 && !ctx->profiling &&
                       lags < (ctx->precision == TGA_PRECISION_FP16_TC ? 4e9 : 6e8);
     if (fork) CK(cudaEventRecord(ctx->forked, st));
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-      const cudaStream_t gs = fork && gi > 0 ? ctx->sides[gi - 1].stream : st;
-      if (gs != st) CK(cudaStreamWaitEvent(gs, ctx->forked, 0));
-      enqueue_codes(ctx, groups[gi], gbufs[gi], gs);
-      enqueue_group(ctx, groups[gi], gbufs[gi], src, d_fc, nb, opt->center_freq, opt->cn0, chip_width_of(fs),
-                    gout[gi], gs);
-      if (gs != st) CK(cudaEventRecord(ctx->sides[gi - 1].joined, gs));
+    try {
+      for (size_t gi = 0; gi < groups.size(); ++gi) {
+        const cudaStream_t gs = fork && gi > 0 ? ctx->sides[gi - 1].stream : st;
+        if (gs != st) CK(cudaStreamWaitEvent(gs, ctx->forked, 0));
+        enqueue_codes(ctx, groups[gi], gbufs[gi], gs);
+        enqueue_group(ctx, groups[gi], gbufs[gi], src, d_fc, nb, opt->center_freq, opt->cn0, chip_width_of(fs),
+                      gout[gi], gs);
+        if (gs != st) CK(cudaEventRecord(ctx->sides[gi - 1].joined, gs));
+      }
+      for (size_t gi = 1; fork && gi < groups.size(); ++gi) CK(cudaStreamWaitEvent(st, ctx->sides[gi - 1].joined, 0));
+    } catch (...) {
+      // a launch failed between fork and join: the next call uses the same
+      // buffers on `stream` alone
+      for (const tga_ctx::Side& sd : ctx->sides) cudaStreamSynchronize(sd.stream);
+      throw;
     }
-    for (size_t gi = 1; fork && gi < groups.size(); ++gi) CK(cudaStreamWaitEvent(st, ctx->sides[gi - 1].joined, 0));
   };
   if (groups.size() > 1 && !ctx->forked) CK(cudaEventCreateWithFlags(&ctx->forked, cudaEventDisableTiming));
   while (ctx->sides.size() + 1 < groups.size()) {
