@@ -77,6 +77,7 @@
 
 #include "engine.h"
 #include "pfa_common.cuh"
+#include "tc_steps.h"
 
 namespace tga {
 
@@ -281,10 +282,11 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t phase) {
 }
 // Two phases at once: a test costs 150 to 300 cycles from issue to answer even
 // when its phase has long completed, so both go out before either is looked at.
+// A phase that its test saw complete is not tested again.
 __device__ __forceinline__ bool warp_wait2(uint32_t bar0, uint32_t phase0, uint32_t bar1, uint32_t phase1) {
   const uint32_t a = mbar_try_wait(bar0, phase0), b = mbar_try_wait(bar1, phase1);
   if (__all_sync(0xffffffffu, a & b)) return true;
-  return __all_sync(0xffffffffu, bounded_wait(bar0, phase0) && bounded_wait(bar1, phase1)) != 0;
+  return __all_sync(0xffffffffu, (a || bounded_wait(bar0, phase0)) && (b || bounded_wait(bar1, phase1))) != 0;
 }
 
 // Per code length: NB blocks of 2 x 32 columns (h, 31-digit) in D1; H2 / B3
@@ -499,6 +501,7 @@ struct Units {
 // s / NCH; a barrier of a chain is in phase (s / NCH) & 1.
 template <class T>
 struct Bars {
+  using Turn = A2Turn<T::NCH, T::A2S>;
   // byte offsets from the CTA's first mbarrier
   static constexpr uint32_t PER = 8 * T::NCH;
   static constexpr uint32_t PROD = 0;         // P1 -> M1: the chain's products are stored (every product warp)
@@ -508,7 +511,8 @@ struct Bars {
   static constexpr uint32_t DFREE = 4 * PER;  // P4 -> M1: D is read (the chain's TMEM warps)
   static constexpr uint32_t A1 = 5 * PER;     // A1's first K steps are in TMEM (4 warps, once)
   static constexpr uint32_t CODE = A1 + 8;    // code block n (slot n % SLOTS) has landed
-  static constexpr int COUNT = 5 * T::NCH + 1 + T::SLOTS;
+  static constexpr uint32_t AFREE = CODE + 8 * T::SLOTS;  // M2 of the region's step done (commit): the region is free
+  static constexpr int COUNT = 5 * T::NCH + 1 + T::SLOTS + Turn::REGION_BARS;
 };
 
 // The M1 warp's thread.  M1 of step s needs its products and the D region that
@@ -633,6 +637,7 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
     }
     mbar_init(bars + Br::A1, 4);
     for (uint32_t x = 0; x < 8 * T::SLOTS; x += 8) mbar_init(bars + Br::CODE + x, 1);
+    for (int r = 0; r < Br::Turn::REGION_BARS; ++r) mbar_init(bars + Br::AFREE + 8u * (uint32_t)r, 1);
   }
   for (int i = tid; i < (T::A1_BYTES + T::B2_BYTES) / 16; i += T::THREADS)
     st_shared(A1 + 16u * (uint32_t)i, __ldg(p.mats + i));
@@ -748,8 +753,9 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
     };
     // ---- M2, by the chain's first warp ----
     const uint64_t db2 = desc_sw128(B2);
-    auto m2 = [&](auto xc, uint32_t region) {
+    auto m2 = [&](auto xc, int reg) {
       constexpr int cx = decltype(xc)::value;
+      const uint32_t region = (uint32_t)(reg * T::A2_COLS);
 #pragma unroll
       for (int k = 0; k < NB; ++k)
 #pragma unroll
@@ -758,6 +764,7 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
                      tmem + region + (uint32_t)(T::A2_COL + 32 * k + 8 * ks),
                      db2 + (uint64_t)(2 * ks), idesc_f16(64, false), ks > 0 ? 1u : 0u);
       mma_commit(bars + Br::M2 + 8u * cx);
+      if (Br::Turn::REGION_BARS) mma_commit(bars + Br::AFREE + 8u * (uint32_t)reg);
     };
     // ---- P4: the warp's 1 / PARTS of the outputs t2 of every block, for the
     // thread's row; two adjacent outputs are one packed value ----
@@ -841,31 +848,27 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
         }
 #pragma unroll 1
         for (int blk = 0; blk < B; ++blk, ++use) {
-          // the step's A2 is free when step s - A2S, of chain x - A2S, has its D2
-          // (before the first such step: the phase ahead of the barrier's first);
-          // with two chains and two regions that is this chain's own last step
-          if (T::A2S < T::NCH) {
-            const int y = x >= T::A2S ? x - T::A2S : x - T::A2S + T::NCH;
-            ok = warp_wait2(bar + Br::M1, use & 1u, bars + Br::M2 + 8u * (uint32_t)y,
-                            (use & 1u) ^ (x >= T::A2S ? 0u : 1u));
-          } else {
+          // D1 is there, and the step's A2 is free (A2Turn)
+          const int step = (int)use * T::NCH + x, reg = Br::Turn::region(step);
+          if (Br::Turn::WAITS)
+            ok = warp_wait2(bar + Br::M1, use & 1u,
+                            bars + (Br::Turn::REGION_BARS ? Br::AFREE : Br::M2) + 8u * (uint32_t)Br::Turn::bar(step),
+                            Br::Turn::parity(step));
+          else
             ok = warp_wait(bar + Br::M1, use & 1u);
-          }
-          const uint32_t region =
-              T::A2S == 1 ? 0u : (T::NCH % 2 == 0 ? (uint32_t)(x & 1) : (use + (uint32_t)x) & 1u) * T::A2_COLS;
           if (!ok) break;
           tc_fence_after();
-          p2(region);
+          p2((uint32_t)(reg * T::A2_COLS));
           if (warp == x * T::CHAIN_WARPS) {
             if (!(ok = warp_wait(bar + Br::A2, use & 1u))) break;
             tc_fence_after();
             if (elect_one()) {
               if (x == 0)
-                m2(std::integral_constant<int, 0>(), region);
+                m2(std::integral_constant<int, 0>(), reg);
               else if (x == 1)
-                m2(std::integral_constant<int, 1>(), region);
+                m2(std::integral_constant<int, 1>(), reg);
               else
-                m2(std::integral_constant<int, T::NCH - 1>(), region);
+                m2(std::integral_constant<int, T::NCH - 1>(), reg);
             }
             __syncwarp();
           }
@@ -882,6 +885,13 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
           }
         }
       }
+    }
+    // drain: the commit on a region's barrier that no later step waits for (of
+    // the CTA's n steps the last ones of every region)
+    if (Br::Turn::REGION_BARS > 0 && ok && use > 0 && warp == x * T::CHAIN_WARPS) {
+      const int n = ((int)use - (x < s ? 1 : 0)) * T::NCH + s, last = ((int)use - 1) * T::NCH + x;
+      if (last >= n - T::A2S)
+        ok = warp_wait(bars + Br::AFREE + 8u * (uint32_t)Br::Turn::region(last), (uint32_t)(last / T::A2S) & 1u);
     }
   } else if (warp < T::M1_WARP) {
     // ---------------- P1: FP16 products ----------------
