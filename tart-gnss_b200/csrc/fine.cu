@@ -26,6 +26,7 @@
 
 #include <cstdint>
 
+#include "chip_index.h"
 #include "engine.h"
 
 namespace tga {
@@ -44,8 +45,7 @@ constexpr int kScanAnt = 24;      // antennas of the scan's tile
 __device__ __forceinline__ void replica(const int8_t* __restrict__ seq, int L, double T, double inv_sigma, double t,
                                         float& c, float& c1, float& c2) {
   const double k = floor(t / T);
-  int kk = (int)(k - floor(k / (double)L) * (double)L);
-  kk = kk < 0 ? kk + L : kk >= L ? kk - L : kk;
+  const int kk = chip_index(k, L);
   auto wrap = [&](int m) -> int { return m < 0 ? m + L : m >= L ? m - L : m; };  // L >= 1023
   c = (float)__ldg(seq + kk);
   c1 = 0.f;
