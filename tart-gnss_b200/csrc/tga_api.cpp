@@ -1621,6 +1621,10 @@ void fine_sums(tga_ctx* ctx, const uint8_t* d_bits, size_t A, size_t row_bytes, 
   }
 }
 
+// Most points of one call's frequency scans, over all its tasks (they are
+// numbered in 32 bits, and each is a row of sums on device and host).
+constexpr size_t kMaxScanPoints = 65535;
+
 // R of every point of the scans, normalised by the window length: out[point][antenna]
 void fine_scan(tga_ctx* ctx, const uint8_t* d_bits, size_t A, size_t row_bytes, const double* d_mean,
                const std::vector<FineScan>& scans, size_t points, std::vector<cplx>& out) {
@@ -1779,7 +1783,10 @@ int tga_fine_acquire(tga_ctx* ctx, const uint8_t* h_bits, size_t n_ant, size_t r
       const double win = (double)tasks[i].length / fs;
       const double df = 0.25 / win;
       const double hw = o.scan_hw == 0.0 ? 150.0 + 1.0 / win : o.scan_hw;
-      const int K = hw < 0 ? 0 : (int)std::ceil(hw / df);
+      const double half = hw < 0 ? 0.0 : std::ceil(hw / df);
+      if (!((double)points + 2.0 * half + 1.0 <= (double)kMaxScanPoints))
+        throw std::runtime_error("the frequency scans take more than 65535 points");
+      const int K = (int)half;
       nscan[i] = K;
       FineScan sc;
       sc.task = fine_task(jobs[i], fs, tasks[i].code_phase, tasks[i].frequency, (int)points);

@@ -24,3 +24,17 @@ def test_code_phase_far_away(const, prn, period):
             ctx.fine_acquire(bits, FS, [(const, prn, tau, IF, 0, N)])
         p1, _, _ = ctx.fine_eval(bits, FS, const, prn, 1234.0, IF, 0, N)
         assert abs(p1 - p0) <= 1e-12 * p0
+
+
+@pytest.mark.parametrize("half_widths", [[2.1e6], [1.3e6, 1.3e6], [1e12], [float("inf")]])
+def test_too_many_scan_points(half_widths):
+    """More than 65535 points over the tasks of a call (steps of 1 / (4 T), 62.5
+    Hz for 4 ms) are refused, and the context works on."""
+    n = 65472
+    bits = np.random.default_rng(4).integers(0, 256, size=(1, n // 8), dtype=np.uint8)
+    tasks = [(tga.GPS, 9 + i, 1234.0, IF, 0, n) for i in range(len(half_widths))]
+    with tga.Context(0) as ctx:
+        with pytest.raises(tga.TgaError):
+            ctx.fine_acquire(bits, FS, tasks, scan_half_width_hz=half_widths[0])
+        res, _ = ctx.fine_acquire(bits, FS, tasks, scan_half_width_hz=600.0)
+        assert all(r["power"] >= r["power_start"] > 0 for r in res)
