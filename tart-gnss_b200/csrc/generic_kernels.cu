@@ -323,12 +323,16 @@ __global__ void select_second_kernel(const float* __restrict__ corr, const unsig
   __shared__ float s_peak;
   if (threadIdx.x < 32) {
     // a bin's row is [c,-c]'s only when strictly stronger; the last bin of the
-    // largest value wins
+    // largest value wins.  A NaN is never above another value, and nothing is
+    // above a NaN in bin 0.
     unsigned long long best = 0ull;  // (value bits, bin)
     for (int b = threadIdx.x; b < nb; b += 32) {
-      const unsigned pa = (unsigned)(keys[2 * b] >> 32), pB = (unsigned)(keys[2 * b + 1] >> 32);
-      const unsigned long long k = ((unsigned long long)max(pa, pB) << 32) | (unsigned)b;
-      best = k > best ? k : best;
+      const float pa = __uint_as_float((unsigned)(keys[2 * b] >> 32));
+      const float pB = __uint_as_float((unsigned)(keys[2 * b + 1] >> 32));
+      const float pr = pB > pa ? pB : pa;
+      const unsigned v = pr >= 0.f ? __float_as_uint(pr) : b == 0 ? 0xffffffffu : 0u;
+      const unsigned long long k = ((unsigned long long)v << 32) | (unsigned)b;
+      if (pr >= 0.f || v != 0u) best = k > best ? k : best;
     }
     for (int o = 16; o > 0; o >>= 1) {
       const unsigned long long t = __shfl_xor_sync(0xffffffffu, best, o);
@@ -337,10 +341,10 @@ __global__ void select_second_kernel(const float* __restrict__ corr, const unsig
     if (threadIdx.x == 0) {
       const int b = (int)(unsigned)best;
       const unsigned long long ka = keys[2 * b], kb = keys[2 * b + 1];
-      const bool useB = (unsigned)(kb >> 32) > (unsigned)(ka >> 32);
+      const bool useB = __uint_as_float((unsigned)(kb >> 32)) > __uint_as_float((unsigned)(ka >> 32));
       s_q = 2 * b + (useB ? 1 : 0);
       s_idx = (int)(unsigned)((useB ? kb : ka) & 0xffffffffu);
-      s_peak = __uint_as_float((unsigned)(best >> 32));
+      s_peak = __uint_as_float((unsigned)((useB ? kb : ka) >> 32));
     }
   }
   __syncthreads();
