@@ -55,7 +55,9 @@ __device__ __forceinline__ void sincos_phase(float ph, float* sn, float* cs) {
   const double th = x * kQuarters[0];
   const double tl = fma(x, kQuarters[1], fma(x, kQuarters[0], -th));
   double t = (th - 4.0 * rint(0.25 * th)) + tl;  // whole turns off
-  if (fabsf(ph) >= 1e30f) t = 0.0 * x;           // no phase: any bounded value, NaN for infinities
+  // (from 3e31 on tl has no bits below a turn, and q needs |t| < 2^51: any
+  // bounded value, NaN for infinities)
+  if (fabsf(ph) >= 3e31f) t = 0.0 * x;
   const double big = t + 6755399441055744.0;
   const int q = __double2loint(big);
   const double r = t - (big - 6755399441055744.0), z = r * r;
