@@ -223,7 +223,8 @@ struct RfiBufs {
   unsigned* hist;               // [n_ant][2][kRfiDigits]
   unsigned long long* prefix;   // [n_ant]: the digits found, in the end the median's bits
   unsigned* rank;               // [n_ant]: rank among the bins that share the prefix
-  unsigned* n_list;             // [n_ant]
+  unsigned* n_same;             // [n_ant]: bins that share the prefix
+  unsigned* n_list;             // [n_ant]: of them in the list
   unsigned long long* list;     // [n_ant][kRfiList]
   unsigned* count;              // [n_ant] candidate lines found
   long long* bins;              // [n_ant][cap]

@@ -16,6 +16,7 @@
 //   * the autocorrelation at lags 1, 3 and 16 (rfi.rs:84-87) exactly from
 //     popcounts: sum z_i z_{i+L} = sum s s' - m (sum s_head + sum s_tail)
 //     + (n - L) m^2 with sum s s' = (n - L) - 2 popcount(b_i xor b_{i+L}).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,10 +30,10 @@ namespace tga {
 namespace {
 
 // the digit holding rank[a] among kRfiDigits counts, one block per antenna:
-// narrows the prefix and the rank
+// narrows the prefix and the rank, and says how many bins share the prefix
 __global__ void __launch_bounds__(256) rfi_select_kernel(const unsigned* __restrict__ hist, int digit, int shift,
                                                          unsigned rank0, unsigned long long* __restrict__ prefix,
-                                                         unsigned* __restrict__ rank) {
+                                                         unsigned* __restrict__ rank, unsigned* __restrict__ n_same) {
   __shared__ unsigned part[256];
   constexpr int PER = kRfiDigits / 256;
   const int a = blockIdx.x, t = threadIdx.x;
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(256) rfi_select_kernel(const unsigned* __restr
     while (cum + h[d] <= r) cum += h[d++];
     prefix[a] = (digit == 0 ? 0ull : prefix[a]) | ((unsigned long long)(t * PER + d) << shift);
     rank[a] = r - cum;
+    n_same[a] = h[d];
   }
 }
 
@@ -95,37 +97,46 @@ __global__ void __launch_bounds__(256) rfi_hist_kernel(const double* __restrict_
     if (sh[i]) atomicAdd(hist + ((size_t)a * 2 + 1) * kRfiDigits + i, sh[i]);
 }
 
-// the bins that share both digits, and their number (it may exceed the list)
+// the bins that share both digits, where the list holds them
 __global__ void __launch_bounds__(256) rfi_gather_kernel(const double* __restrict__ p, unsigned half,
                                                          const unsigned long long* __restrict__ prefix,
+                                                         const unsigned* __restrict__ n_same,
                                                          unsigned* __restrict__ n_list,
                                                          unsigned long long* __restrict__ list) {
   const int a = blockIdx.y;
+  if (n_same[a] > (unsigned)kRfiList) return;
   const unsigned long long pre = prefix[a] >> kRfiShift1;
   for_powers(p, half, a, [&](unsigned long long u) {
-    if (u >> kRfiShift1 == pre) {
-      const unsigned i = atomicAdd(n_list + a, 1u);
-      if (i < (unsigned)kRfiList) list[(size_t)a * kRfiList + i] = u;
-    }
+    if (u >> kRfiShift1 == pre) list[(size_t)a * kRfiList + atomicAdd(n_list + a, 1u)] = u;
   });
 }
 
-// the element of rank[a] among the gathered bins, one block per antenna.  More
-// bins than the list holds (many equal powers): three more digits over the
-// whole row by this block.
-__global__ void __launch_bounds__(256) rfi_median_kernel(const double* __restrict__ p, unsigned half,
-                                                         const unsigned* __restrict__ n_list,
-                                                         const unsigned long long* __restrict__ list,
-                                                         const unsigned* __restrict__ rank,
-                                                         unsigned long long* __restrict__ prefix) {
+// The element of rank[a] among the gathered bins, one cluster per antenna: its
+// first CTA ranks the list.  More bins than the list holds (a constant row, whose
+// powers are all 0, or one with few samples off): three more digits over the
+// whole row by the cluster, each CTA counting its share and summing an eighth
+// of the digits over all.  One row of 818400 equal powers: the scan of one
+// antenna takes 246 us; with one CTA for the digits, and the bins gathered
+// before they were counted, 1074.
+constexpr int kMedianCtas = 8, kMedianThreads = kRfiDigits / kMedianCtas;
+
+__global__ void __cluster_dims__(kMedianCtas, 1, 1) __launch_bounds__(kMedianThreads)
+    rfi_median_kernel(const double* __restrict__ p, unsigned half, const unsigned* __restrict__ n_same,
+                      const unsigned long long* __restrict__ list, const unsigned* __restrict__ rank,
+                      unsigned long long* __restrict__ prefix) {
+  namespace cg = cooperative_groups;
   __shared__ unsigned sh[kRfiDigits];
+  __shared__ unsigned s_warp[kMedianThreads / 32], s_total;
   __shared__ unsigned long long s_pre;
   __shared__ unsigned s_rank;
-  const int a = blockIdx.x;
-  const unsigned n = n_list[a], r = rank[a];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int a = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned me = cluster.block_rank(), n = n_same[a];
   if (n <= (unsigned)kRfiList) {
+    if (me != 0) return;
+    const unsigned r = rank[a];
     const unsigned long long* l = list + (size_t)a * kRfiList;
-    for (unsigned i = threadIdx.x; i < n; i += 256) {
+    for (unsigned i = tid; i < n; i += kMedianThreads) {
       unsigned less = 0, same = 0;
       for (unsigned k = 0; k < n; ++k) {
         less += l[k] < l[i] ? 1u : 0u;
@@ -135,31 +146,68 @@ __global__ void __launch_bounds__(256) rfi_median_kernel(const double* __restric
     }
     return;
   }
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     s_pre = prefix[a];
-    s_rank = r;
+    s_rank = rank[a];
   }
-  const double* row = p + (size_t)a * half;
+  const double2* row = reinterpret_cast<const double2*>(p + (size_t)a * half);
+  constexpr unsigned stride = kMedianCtas * kMedianThreads;
   for (int shift = kRfiShift1 - 13; shift > -13; shift -= 13) {
     const int lo = shift < 0 ? 0 : shift, width = shift < 0 ? 13 + shift : 13;
-    for (int i = threadIdx.x; i < kRfiDigits; i += 256) sh[i] = 0;
+    for (int i = tid; i < kRfiDigits; i += kMedianThreads) sh[i] = 0;
     __syncthreads();
-    const unsigned long long pre = s_pre >> (lo + width);
-    for (unsigned k = threadIdx.x; k < half; k += 256) {
-      const unsigned long long u = (unsigned long long)__double_as_longlong(__ldg(row + k));
-      if (u >> (lo + width) == pre) atomicAdd(&sh[(u >> lo) & ((1u << width) - 1)], 1u);
+    const unsigned long long pre = s_pre;
+    const unsigned left = s_rank;
+    // equal digits of a warp are counted at once
+    auto add = [&](double v, bool on) {
+      const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+      const unsigned d = on && u >> (lo + width) == pre >> (lo + width) ? (unsigned)(u >> lo) & ((1u << width) - 1) : ~0u;
+      const unsigned d0 = __shfl_sync(0xffffffffu, d, 0);
+      if (__all_sync(0xffffffffu, d == d0)) {
+        if (lane == 0 && d != ~0u) atomicAdd(&sh[d], 32u);
+      } else if (d != ~0u) {
+        atomicAdd(&sh[d], 1u);
+      }
+    };
+    for (unsigned w = me * kMedianThreads + 32 * warp; w < half / 2; w += 4 * stride) {
+      double2 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[i] = make_double2(0.0, 0.0);
+        if (w + lane + i * stride < half / 2) v[i] = __ldg(row + w + lane + i * stride);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool on = w + lane + i * stride < half / 2;
+        add(v[i].x, on);
+        add(v[i].y, on);
+      }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned left = s_rank;
-      int d = 0;
-      while (sh[d] <= left) left -= sh[d++];
-      s_rank = left;
-      s_pre |= (unsigned long long)d << lo;
+    cluster.sync();
+    // digit me kMedianThreads + tid of the whole row, and the counts up to it
+    unsigned c = 0;
+#pragma unroll
+    for (int q = 0; q < kMedianCtas; ++q) c += *cluster.map_shared_rank(&sh[me * kMedianThreads + tid], q);
+    unsigned upto = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
     }
+    if (lane == 31) s_warp[warp] = upto;
     __syncthreads();
+    for (int q = 0; q < warp; ++q) upto += s_warp[q];
+    if (tid == kMedianThreads - 1) s_total = upto;
+    cluster.sync();
+    for (unsigned q = 0; q < me; ++q) upto += *cluster.map_shared_rank(&s_total, q);
+    if (left < upto && left >= upto - c) {  // one thread of the cluster
+      for (int q = 0; q < kMedianCtas; ++q) {
+        *cluster.map_shared_rank(&s_pre, q) = pre | (unsigned long long)(me * kMedianThreads + tid) << lo;
+        *cluster.map_shared_rank(&s_rank, q) = left - (upto - c);
+      }
+    }
+    cluster.sync();
   }
-  if (threadIdx.x == 0) prefix[a] = s_pre;
+  if (me == 0 && tid == 0) prefix[a] = s_pre;
 }
 
 __global__ void rfi_peaks_kernel(const double* __restrict__ p, long long half, const unsigned long long* __restrict__ floor_bits,
@@ -245,11 +293,12 @@ cudaError_t rfi_scan_device(const uint8_t* d_bits, int n_ant, size_t row_bytes, 
   // median bin power: rank half / 2 (rfi.rs:110-111)
   const unsigned h = (unsigned)half;
   const dim3 g((unsigned)std::min<long long>(std::max(32, 8 * num_sms / n_ant), (half + 2047) / 2048), (unsigned)n_ant);
-  rfi_select_kernel<<<n_ant, 256, 0, st>>>(b.hist, 0, kRfiShift0, h / 2, b.prefix, b.rank);
+  rfi_select_kernel<<<n_ant, 256, 0, st>>>(b.hist, 0, kRfiShift0, h / 2, b.prefix, b.rank, b.n_same);
   rfi_hist_kernel<<<g, 256, 0, st>>>(b.p, h, b.prefix, b.hist);
-  rfi_select_kernel<<<n_ant, 256, 0, st>>>(b.hist, 1, kRfiShift1, 0u, b.prefix, b.rank);
-  rfi_gather_kernel<<<g, 256, 0, st>>>(b.p, h, b.prefix, b.n_list, b.list);
-  rfi_median_kernel<<<n_ant, 256, 0, st>>>(b.p, h, b.n_list, b.list, b.rank, b.prefix);
+  rfi_select_kernel<<<n_ant, 256, 0, st>>>(b.hist, 1, kRfiShift1, 0u, b.prefix, b.rank, b.n_same);
+  rfi_gather_kernel<<<g, 256, 0, st>>>(b.p, h, b.prefix, b.n_same, b.n_list, b.list);
+  rfi_median_kernel<<<dim3(kMedianCtas, (unsigned)n_ant), kMedianThreads, 0, st>>>(b.p, h, b.n_same, b.list, b.rank,
+                                                                                  b.prefix);
   rfi_peaks_kernel<<<dim3(256, (unsigned)n_ant), 256, 0, st>>>(b.p, half, b.prefix, 15.0, cap, b.count, b.bins,
                                                                b.excess);
   rfi_acf_kernel<<<dim3(64, (unsigned)n_ant), 256, 0, st>>>(d_bits, row_bytes, n, b.acf);

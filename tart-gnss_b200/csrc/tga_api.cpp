@@ -1932,6 +1932,7 @@ int tga_rfi_scan(tga_ctx* ctx, const uint8_t* h_bits, size_t n_ant, size_t row_b
     rb.hist = (unsigned*)ctx->buf("rfi.hist", A * 2 * kRfiDigits * sizeof(unsigned));
     rb.prefix = (unsigned long long*)ctx->buf("rfi.prefix", A * 8);
     rb.rank = (unsigned*)ctx->buf("rfi.rank", A * sizeof(unsigned));
+    rb.n_same = (unsigned*)ctx->buf("rfi.n_same", A * sizeof(unsigned));
     rb.n_list = (unsigned*)ctx->buf("rfi.n_list", A * sizeof(unsigned));
     rb.list = (unsigned long long*)ctx->buf("rfi.list", A * kRfiList * 8);
     rb.count = (unsigned*)ctx->buf("rfi.count", A * sizeof(unsigned));
