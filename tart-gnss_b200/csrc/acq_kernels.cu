@@ -132,7 +132,7 @@ __device__ __forceinline__ float2 carrier(const FrontParams& p, int n, double nd
 // when every antenna computed them, 1.9 ms).
 template <bool BITS, bool GROUP>
 __global__ void __launch_bounds__(256) frontend_kernel(FrontParams p) {
-  extern __shared__ float2 fsm[];
+  extern __shared__ __align__(16) float2 fsm[];
   const int S = p.S, P = p.P, Lc = p.Lc;
   const int grp = blockIdx.y / p.nb, bin = blockIdx.y - grp * p.nb;
   const int ant0 = GROUP ? grp * p.n_grp : grp, ant1 = GROUP ? min(ant0 + p.n_grp, p.src.n_ant) : ant0 + 1;
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(NT, MINB) pfa_kernel(PfaParams p) {
   constexpr int COLS = G::COLS, LC = G::LC, NC = G::NC;
   constexpr bool INV = (MODE == CORR || MODE == SECOND || MODE == CAND);
   constexpr bool ARGMAX = (MODE == CORR || MODE == CAND);
-  extern __shared__ float2 buf[];
+  extern __shared__ __align__(16) float2 buf[];
   __shared__ unsigned long long s_key;
   __shared__ unsigned int s_p2;
   __shared__ unsigned int s_floor;

@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(Tc<M, NCB>::THREADS, 1) pfa_tc_kernel(const __
   using U = TcUnits<M>;
   using Br = Bars<T>;
   constexpr int NB = T::NB, RES = T::RES, GR = U::GR;
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t s_bar[Br::COUNT];
   __shared__ uint32_t s_tmem;
   // 32-bit shared addresses of the regions, from a 1024-byte boundary

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kPassThreads) pass64_kernel(const double2* __r
                                                               double2* __restrict__ out,
                                                               const double2* __restrict__ tw, unsigned L,
                                                               unsigned Ns) {
-  extern __shared__ double2 s_out[];
+  extern __shared__ __align__(16) double2 s_out[];
   const unsigned LR = L / R, j = blockIdx.x * kPassThreads + threadIdx.x;
   const size_t seq = (size_t)blockIdx.y * L;
   double2 v[R];

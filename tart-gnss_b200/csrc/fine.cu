@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kFineThreads) fine_scan_kernel(const uint8_t* 
                                                                  size_t row_bytes, const double* __restrict__ mean,
                                                                  const FineScan* __restrict__ tasks,
                                                                  double* __restrict__ out) {
-  extern __shared__ float2 s_mem[];
+  extern __shared__ __align__(16) float2 s_mem[];
   float2* s_w = s_mem;                               // [kScanSub][kScanK]
   float2* s_s = s_mem + (size_t)kScanSub * kScanK;   // [kScanSub][kScanAnt / 2]: two antennas' samples
   const FineScan sc = tasks[blockIdx.y];

@@ -97,7 +97,7 @@ constexpr int kGenThreads = 128;
 template <int R, bool STAGE>
 __global__ void __launch_bounds__(kGenThreads) pass32_kernel(const float2* __restrict__ in, float2* __restrict__ out,
                                                              const float2* __restrict__ tw, unsigned L, unsigned Ns) {
-  extern __shared__ float2 s_out[];
+  extern __shared__ __align__(16) float2 s_out[];
   const unsigned LR = L / R, j = blockIdx.x * kGenThreads + threadIdx.x;
   const size_t seq = (size_t)blockIdx.y * L;
   if (j < LR) {

@@ -62,7 +62,7 @@ __device__ __forceinline__ float2 phasor_turns(double t) {
 // per tap 24 antennas x 201 bins x 10 blocks of 10 periods take 5.0 ms instead
 // of 5.4, one antenna x 21 bins x 10 blocks of one period 22.7 us instead of 28.
 __global__ void __launch_bounds__(256) nc_frontend_kernel(NcFrontParams p) {
-  extern __shared__ float2 fsm[];
+  extern __shared__ __align__(16) float2 fsm[];
   const int S = p.S, P = p.P, Lc = p.Lc;
   const int ab = blockIdx.y / p.B, blk = blockIdx.y - ab * p.B;
   const int ant_slot = ab / p.nb, bin = ab - ant_slot * p.nb;
@@ -219,7 +219,7 @@ template <int M, int BC, int NT, int MINB, int MODE>
 __global__ void __launch_bounds__(NT, MINB) nc_correlate_kernel(NcParams p) {
   using G = Geo<M>;
   constexpr int COLS = G::COLS, LC = G::LC, NC = G::NC;
-  extern __shared__ float2 buf[];
+  extern __shared__ __align__(16) float2 buf[];
   float* acc = reinterpret_cast<float*>(buf + BC * LC);
   __shared__ unsigned long long s_key;
   __shared__ unsigned int s_p2;
