@@ -21,8 +21,8 @@
 // Frequency-domain arrays use the digit layout [k31][kM][k33]; time-domain
 // lag digits map to natural lags by the Chinese remainder theorem.
 //
-// Generic path (any N): the reference algorithm on the GPU, with Bluestein
-// FFTs of length N built on a power-of-two Stockham FFT.
+// Generic path (any N, generic_kernels.cu): the reference algorithm on the GPU,
+// with mixed-radix FFTs of length N, or Bluestein's where N has a large prime.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 

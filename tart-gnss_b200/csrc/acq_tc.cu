@@ -46,8 +46,10 @@
 // and P4, so that one chain's P4 runs beside the other's P2, and one warp that
 // issues M1 and fetches the code blocks.  M2 is issued by the first of its
 // chain's warps: a thread's barrier test queues behind its own MMAs, so one
-// issuer for both stages would see A2 late (measured: 1000 cycles).  Every wait is bounded (1 s): on expiry a role sets *err, drains (again bounded)
-// and leaves its loop.
+// issuer for both stages would see A2 late (measured: 1000 cycles).  Which
+// barrier tells that an A2 region is free is tc_steps.h's.  Every wait is
+// bounded (1 s): on expiry a role sets *err, drains (again bounded) and leaves
+// its loop.
 //
 // What bounds it (Lc = 10230, per step, of about 2550 cycles measured over the
 // whole 24-antenna search): the shared-memory data path, about 1600 cycles (P1
@@ -178,10 +180,9 @@ __device__ __forceinline__ void mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uin
       "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc), "r"(z), "r"(z), "r"(z), "r"(z)
       : "memory");
 }
-// True in one lane of a converged warp.  tcgen05.mma takes its descriptors from
-// uniform registers: behind elect.sync the compiler keeps them there, behind a
-// lane test it moves them over before every MMA (measured at M = 128, N = 64,
-// K = 16 with A in TMEM: 54 cycles per MMA behind the lane test, 36 here).
+// True in one lane of a converged warp.  Measured at M = 128, N = 64, K = 16
+// with A in TMEM: an MMA issues every 54 cycles behind a lane test, every 36
+// behind elect.sync.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile(

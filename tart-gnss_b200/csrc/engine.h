@@ -91,7 +91,7 @@ cudaError_t launch_forward_z(const PolyClass& pc, int n_ab, float2* d_z, int num
 // (launch_tc_pack's layout and scale, tc_z_scale) from shared memory
 cudaError_t launch_forward_z_tc(const PolyClass& pc, int n_ab, float2* d_z, void* d_z16, const void* d_map,
                                 float z16_scale, int num_sms, cudaStream_t st);
-// d_map of launch_forward_z_tc for chip count 1023 M: per FP16 unit four
+// d_map of launch_forward_z_tc for chip count 1023 M: per FP16 unit eight
 // 16-bit offsets into the transformed sequence (0xffff: zero), host-built
 std::vector<uint16_t> tc_unit_map(int M);
 // launch_forward_seqs that also writes the tensor-core FP16 operands
@@ -139,18 +139,19 @@ cudaError_t launch_tc_candidates(const SearchDims& dims, int n_hyp, const unsign
 // (comparisons only) and must be zeroed before the launch; *d_err is set
 // non-zero when a bounded wait on the tensor cores expired.
 size_t tc_operand_bytes(const PolyClass& pc, long long n_seq);
-// the three inverse-DFT matrices of class M in the correlator's shared-memory
-// layouts (FP16), to be uploaded once and passed as d_bmat
+// the two inverse-DFT matrices (DFT-R1 and DFT-31) of class M in the
+// correlator's shared-memory layouts (FP16), to be uploaded once and passed as
+// d_bmat
 std::vector<unsigned char> tc_dft_matrices(int M);
 cudaError_t launch_tc_pack(const PolyClass& pc, const float2* d_src, long long n_seq, bool code, void* d_dst,
                            int num_sms, cudaStream_t st);
-// test_flags bit 0: skip the first MMA batch and its commit (test hook for
+// test_flags bit 0: the first stage issues no MMA and no commit (test hook for
 // the bounded-wait failure path; 0 in normal use)
 cudaError_t launch_correlate_tc(const PolyClass& pc, const SearchDims& dims, const void* d_bmat, const void* d_z16,
                                 const void* d_d16, unsigned long long* d_keys, int* d_err, int test_flags,
                                 int num_sms, cudaStream_t st);
-// the non-coherent search (Lc = 1023): per (antenna, bin) row and PRN the
-// row maximum of |y|^2 summed over B coherent blocks; z16 holds the FP16 Z of
+// the non-coherent search: per (antenna, bin) row and PRN the row maximum of
+// |y|^2 summed over B coherent blocks; z16 holds the FP16 Z of
 // [n_ant * nb][B][S] sequences
 cudaError_t launch_correlate_tc_nc(const PolyClass& pc, const SearchDims& dims, int B, const void* d_bmat,
                                    const void* d_z16, const void* d_d16, unsigned long long* d_keys, int* d_err,

@@ -9,8 +9,9 @@
 //
 // (k < Ns, r < R, W_L = exp(-2 pi i / L)), so after the passes of all
 // factors of L the result is in natural order.  Each pass reads and writes
-// the whole batch, so what bounds a pass is HBM and what counts is their
-// number: the factors are gathered into radices of up to 33 (32; 33 = 3 x 11
+// the whole batch, so what counts is their number (a pass runs at 4 to 6 TB/s,
+// HBM half busy: 7 to 10 warps per SM, which the butterfly's registers allow,
+// wait for their loads): the factors are gathered into radices of up to 33 (32; 33 = 3 x 11
 // and 15 = 3 x 5 without twiddles; 25; 31, ...), one whole butterfly per thread in
 // registers, and the first pass reads the packed bits themselves.  24 rows of
 // 1636800 samples (L = 32 x 25 x 33 x 31): the seven passes of radices 16, 2,

@@ -37,8 +37,14 @@ constexpr int kFineThreads = 256;
 constexpr int kFineChunk = 1024;  // samples per block of the sums
 constexpr int kScanSub = 256;     // samples of the scan's shared-memory tile
 constexpr int kScanTiles = 4;     // tiles per block of the scan
-constexpr int kScanK = 21;        // frequencies of the scan's tile
-constexpr int kScanAnt = 24;      // antennas of the scan's tile
+// frequencies and antennas of the scan's tile, one (frequency, antenna pair) per
+// thread: the default scan of a 10 ms window on the receiver's 24 antennas fills
+// 252 of 256.  A narrower scan or fewer antennas leave threads of the products
+// idle, more of either repeats a tile's replicas; against the six sums at every
+// frequency it is still ahead everywhere (4 satellites, 100 ms, 129 frequencies:
+// 1 antenna 20.4 -> 4.1 ms, 9 antennas 33.4 -> 7.0, 25 antennas 54.4 -> 14.5, 48
+// antennas 89 -> 23; one satellite, 10 ms, 2 antennas 478 -> 406 us a call).
+constexpr int kScanK = 21, kScanAnt = 24;
 
 // replica value and its first two derivatives at continuous time t (samples)
 // from the four edges around t: c(t) = seq[k] + sum_m d_m (Phi(u_m) - [u_m >= 0])
@@ -161,7 +167,9 @@ __global__ void __launch_bounds__(kFineThreads) fine_sums_kernel(const uint8_t* 
 // then R[a][k] = sum_n s_a[n] w[n][k] is a small matrix product from shared
 // memory, two antennas and one frequency per thread: 12 satellites x 21
 // frequencies x 24 antennas x 163680 samples took 2.38 ms as 252 evaluations
-// of the six sums, and take 0.39 ms so (half of it the 21 phasors per sample).  FP32 over 32 samples, then f64.
+// of the six sums, and take 0.39 ms so (half of it the 21 phasors per sample).
+// Bound by the shared-memory path (its wavefronts 71 % of peak, issue 52 %).  FP32
+// over 32 samples, then f64.
 __global__ void __launch_bounds__(kFineThreads) fine_scan_kernel(const uint8_t* __restrict__ bits, int n_ant,
                                                                  size_t row_bytes, const double* __restrict__ mean,
                                                                  const FineScan* __restrict__ tasks,

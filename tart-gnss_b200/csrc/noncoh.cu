@@ -445,7 +445,9 @@ __global__ void __launch_bounds__(NT, MINB) nc_correlate_kernel(NcParams p) {
 // (32 PRNs x 21 bins x 10 periods of Lc = 1023: 455 us with one, 367 with two).
 // FEW: fewer residues per CTA for calls whose rows' groups would not give every
 // SM a CTA: a block then takes its stages' latency, not the issue slots of nine
-// warps (second peaks of 32 PRNs over ten periods: 56 us on 64 CTAs, 37 on 256).
+// warps (second peaks of 32 PRNs over ten periods of Lc = 1023: 56 us on 64 CTAs,
+// 37 on 256; whole calls at Lc = 4092, 16 samples a chip, 5 blocks: 1 PRN x 1 bin
+// 174 -> 147 us, 4 x 5 198 -> 184, 8 x 5 247 -> 234; equal from 32 rows on).
 template <int M, bool FEW>
 struct NcCfg;
 template <>

@@ -9,7 +9,8 @@
 //     the non-negative powers (RfiBufs), no sorting.  24 rows of 818400 bins: the
 //     eight histogram passes and their serial digit searches took 0.41 ms;
 //     the first digit is counted where the powers are made, the second and the
-//     gathering of the few bins left are a pass each, 0.08 ms in all;
+//     gathering of the few bins left are a pass each, 0.08 ms in all (rows of
+//     equal powers, which leave too many bins: rfi_median_kernel);
 //   * local maxima p[k] > p[k-1], p[k] >= p[k+1] with 10 log10(p / floor) >
 //     15 dB (rfi.rs:113-123), appended to a per-antenna list that the host
 //     clusters (10 kHz, strongest first, at most 3 lines; rfi.rs:125-139);

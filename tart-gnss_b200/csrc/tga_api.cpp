@@ -8,7 +8,7 @@
 // samples per chip, e.g. 16.368 MHz -- the fused polyphase kernels run.
 // Constellations that share the period, the Doppler grid and the pulse
 // (GPS/SBAS/QZSS; BeiDou/L1C) share one front end.  Anything else runs the
-// generic GPU path (the reference algorithm with Bluestein FFTs).
+// generic GPU path (the reference algorithm with FFTs of the window's length).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -374,9 +374,10 @@ double corr_row_flops(int P) { return fft_flops((double)P) + 9.0 * (double)P; }
 // key of their (antenna, PRN) are re-evaluated in FP32.  kTcKeyKeep =
 // (1 - 2 d)^2 with d = 2^-8 a bound on the FP16 transform's amplitude error
 // at any lag, relative to the largest row amplitude of the (antenna, PRN):
-// the FP16 stages round 5 to 7 times at a unit roundoff of 2^-11, and the
-// largest error measured over the test and benchmark workloads (every code
-// length, drop-in and non-coherent, noise-only cells) is 5.6e-4, 7x below d
+// a term is rounded seven times at a unit roundoff of 2^-11 (Z, the code, their
+// product twice, both DFT matrices, the first stage's output), and the largest
+// error measured over searches of every code length at 6 to 18 samples a chip,
+// drop-in and non-coherent, and the benchmark workloads is 4.6e-4, 8x below d
 // (tga_last_row_peaks reports the keys for that measurement).
 constexpr float kTcKeyKeep = (1.0f - 2.0f / 256.0f) * (1.0f - 2.0f / 256.0f);
 
@@ -553,10 +554,7 @@ GroupBufs prepare_group(tga_ctx* ctx, const ClassGroup& grp, int n_ant, int nb, 
   return b;
 }
 
-// Enqueues the fused pipeline of one class group on the context stream
-// (launches, memsets and the copy of the finalised cells into host_out,
-// pinned memory of n_ant * n_prn CellOut).
-// The part of a class's search that needs no signal.
+// The part of a class's search that needs no signal, on `st`.
 void enqueue_codes(tga_ctx* ctx, const ClassGroup& grp, const GroupBufs& b, cudaStream_t st) {
   const PolyClass& pc = grp.pc;
   const int n_prn = (int)grp.prns.size();
@@ -568,7 +566,9 @@ void enqueue_codes(tga_ctx* ctx, const ClassGroup& grp, const GroupBufs& b, cuda
           [&] { return launch_tc_pack(pc, b.D, (long long)n_prn * 2, true, b.d16, ctx->num_sms, st); });
 }
 
-// The rest of it, after enqueue_codes (and in tensor-core mode after *b.err is 0).
+// The rest of the fused pipeline of one class group, on `st` after enqueue_codes
+// (and in tensor-core mode after *b.err is 0): launches, memsets and the copy of
+// the finalised cells into host_out, pinned memory of n_ant * n_prn CellOut.
 void enqueue_group(tga_ctx* ctx, const ClassGroup& grp, const GroupBufs& b, const SampleSource& src,
                    const double* d_fc, int nb, double center, int want_cn0, int chip_width, CellOut* host_out,
                    cudaStream_t st) {
@@ -770,11 +770,14 @@ int acquire_all_impl(tga_ctx* ctx, const uint8_t* d_bits, size_t n_ant_total, si
     if (ctx->precision == TGA_PRECISION_FP16_TC && !gbufs.empty()) CK(cudaMemsetAsync(gbufs[0].err, 0, sizeof(int), st));
     // The classes share no buffer that one of them writes, apart from the error
     // flag they may all set.  In a short search a stream each lets the small
-    // kernels of one class run beside the others' (one antenna, tensor cores:
-    // 2.81 -> 2.66 ms; a few antennas and PRNs in FP32: 3.08 -> 2.98 ms).  In a
-    // long one the correlators of two lengths would share SMs and their
-    // instruction caches (24 antennas in FP32: 179.9 -> 185.2 ms, 57.1 -> 57.6 with
-    // tensor cores), so it keeps one, as per-kernel timing does.
+    // kernels of one class run beside the others'; in a long one the correlators
+    // of two lengths share SMs and their instruction caches, so it keeps one, as
+    // per-kernel timing does.  One stream's time over a stream each's, by lags:
+    //   FP32   1e8 1.14, 2e8 1.09, 4e8 1.05 to 1.07, 6e8 1.02 to 1.06, 1.0e9 1.02,
+    //          1.8e9 0.995, 3.1e9 1.00, 2.5e10 0.97
+    //   tensor 1.6e8 1.14, 4e8 1.12, 1.0e9 1.09, 2.1e9 1.05, 3.1e9 1.03, 4.2e9 1.05,
+    //          6.3e9 1.01, 8.4e9 1.02, 1.3e10 1.01, 1.7e10 0.99, 2.5e10 0.99
+    // Below the limits every set of code lengths measured gains 1.5 % or more.
     double lags = 0.0;
     for (const auto& g : groups) lags += (double)ants.size() * nb * (double)g.prns.size() * g.pc.P;
     const bool fork = groups.size() > 1 && !ctx->profiling &&

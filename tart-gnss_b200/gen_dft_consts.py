@@ -1,10 +1,8 @@
 #!/usr/bin/env python3
 """Writes csrc/dft_consts.cuh: cos/sin(2 pi m / R) for the odd prime DFT
 lengths R in {3, 5, 11, 31}, evaluated in double precision and rounded once
-to binary32; each table also as (v, v) float2 pairs, the operand form of the
-packed FP32 instructions (__ffma2_rn) that apply one constant to the real and
-imaginary parts of a complex value at once.  And csrc/mixed_radix_consts.cuh:
-the same functions in both precisions for the radices of the mixed-radix FFTs."""
+to binary32.  And csrc/mixed_radix_consts.cuh: the same functions in both
+precisions for the radices of the mixed-radix FFTs."""
 import math
 import os
 
