@@ -509,7 +509,9 @@ typedef struct tga_fine_task {
 typedef struct tga_fine_options {
   double edge_sigma_chips;   /* replica edge smoothing, chips (0 -> 0.1)      */
   double scan_half_width_hz; /* frequency pre-scan +- this around the start
-                                (0 -> 150 Hz + 1/window; < 0 -> no scan)      */
+                                (0 -> 150 Hz + 1/window; < 0 -> no scan), in
+                                steps of 1/(4 window); at most 65535 points
+                                over the tasks of a call                      */
   int32_t max_iter;          /* Newton evaluations (0 -> 20)                  */
   double tol_code_phase;     /* convergence, samples (0 -> 1e-4)              */
   double tol_frequency;      /* convergence, Hz (0 -> 1e-3)                   */
